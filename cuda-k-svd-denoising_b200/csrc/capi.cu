@@ -404,11 +404,10 @@ ksvd_status update_prepare(ksvd_ctx* c, const float* d_patches, int64_t N, float
   KSVD_TRY(wsT(c, "csr_atom_ptr", size_t(2) * K + 1, &w.atom_ptr));
   KSVD_TRY(wsT(c, "csr_entries", size_t(N) * L, &w.entries));
   w.records = nullptr;  // the residual-based sweep needs only the entries
-  float *resid = nullptr, *gw = nullptr;
-  unsigned* sync = nullptr;
+  float* resid = nullptr;
+  void* gw = nullptr;
   KSVD_TRY(wsT(c, "upd_resid", size_t(N) * n, &resid));
-  KSVD_TRY(wsT(c, "upd_partials", ksvd::update_res_partial_floats(n, ctas), &gw));
-  KSVD_TRY(wsT(c, "upd_sync", size_t(2) * K, &sync));
+  KSVD_TRY(ws(c, "upd_partials", ksvd::update_res_scratch_bytes(n, ctas, K), &gw));
   int* last = nullptr;
   KSVD_TRY(wsT(c, "upd_last", size_t(N), &last));
   {
@@ -430,7 +429,6 @@ ksvd_status update_prepare(ksvd_ctx* c, const float* d_patches, int64_t N, float
   g->entries = w.entries;
   g->last = last;
   g->gw = gw;
-  g->sync = sync;
   g->n = n;
   g->K = K;
   g->L = L;

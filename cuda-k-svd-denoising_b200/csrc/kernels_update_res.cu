@@ -18,17 +18,15 @@
 // split over `active` CTAs (about slice_target entries each); each keeps its
 // columns in shared memory (those beyond the capacity are re-read from the
 // residual on every pass).  A power step is one pass over the local columns
-// producing a partial w, then an all-reduce: each CTA writes its partial,
-// arrives on the atom's counter and, once all active CTAs have arrived, sums
-// all partials in the same fixed order, so every CTA holds the same u and
-// takes the same convergence decision.  An atom's CTAs wait for the previous
-// atom's CTAs to finish their residual stores before reading the residual;
-// since those in turn waited for the atom before, every earlier atom of the
-// sweep is complete by then.  CTAs with no entries in an atom skip it.  All
+// producing a partial w, then an all-reduce: each CTA writes its partial (as
+// tagged words, or as a plain row behind a counter) and sums all CTAs'
+// partials in the same fixed order, so every CTA holds the same u and takes
+// the same convergence decision.  A CTA alone on its atom needs no exchange.
+// An atom's CTAs wait for the previous atom's CTAs to finish their residual
+// stores before reading the residual; since those in turn waited for the atom
+// before, every earlier atom of the sweep is complete by then.  CTAs with no entries in an atom skip it.  All
 // waits are bounded.
 #include <cuda_runtime.h>
-
-#include <cstring>
 
 #include "device_util.cuh"
 #include "ksvd_internal.cuh"
@@ -48,24 +46,35 @@ __host__ __device__ inline int ur_n4(int n) { return (n + 3) & ~3; }
 // count is odd, so that the 8 rows a quarter-warp reads with 16-byte loads
 // sit in distinct banks.
 __host__ __device__ inline int ur_es(int n) { return 4 * ((ur_n4(n) / 4) | 1); }
-constexpr int kUrRows = 32;  // reduction rows: 16 column groups + 16 streaming warps
 
-// Shared memory: [cap x es] columns | ent[2][cap] | xold[2][cap] | keep[2][cap] |
-// u[n4] | dold[n4] | dnext[n4] | wred[kUrRows x n4]
-__host__ __device__ inline size_t ur_fixed_bytes(int n) {
-  const int n4 = ur_n4(n);
-  return size_t(n4) * 4 * 3 + size_t(kUrRows) * n4 * 4;
+// Column groups of the w pass, and groups of partials of the all-reduce: the
+// order in which w is summed.
+__host__ __device__ inline int ur_groups(int n) {
+  const int g = kUrThreads / (ur_n4(n) / 4);
+  return g > 16 ? 16 : (g < 1 ? 1 : g);
 }
+
+// Row stride of the transposed u (floats): 16-byte rows in distinct banks.
+__host__ __device__ inline int ur_ft(int n) { return 4 * (((ur_n4(n) / 4 + 3) / 4) | 1); }
+
+// Shared memory: [cap x es] columns | row[2][cap] | xold[2][cap] | slices of the
+// next atoms (int4 [kUrTab]) | transposed u[4][ft] | u[n4] | dold[2][n4] | wsum[n4] |
+// wred[groups x n4] | streamed columns: [16 x n4].  The capacity also decides which columns are
+// streamed, hence the order of their sums; it is the one of a layout of 24
+// bytes a column and 35 rows.
+constexpr int kUrTab = 128;
 
 int update_res_capacity(int n) {
   const size_t per = size_t(ur_es(n)) * 4 + 24;
-  const size_t fixed = ur_fixed_bytes(n);
+  const size_t fixed = size_t(35) * ur_n4(n) * 4;
   if (fixed + per * 16 > kUrSmemMax) return 0;
-  // a multiple of 4 keeps u, dold, dnext and wred (read as float4) 16-byte aligned
   return int((kUrSmemMax - fixed) / per) & ~3;
 }
 
-size_t update_res_smem_bytes(int n, int cap) { return size_t(cap) * (size_t(ur_es(n)) * 4 + 24) + ur_fixed_bytes(n); }
+size_t update_res_smem_bytes(int n, int cap) {
+  return size_t(cap) * (size_t(ur_es(n)) * 4 + 16) + kUrTab * 16 + size_t(4) * ur_ft(n) * 4 +
+         size_t(4 + ur_groups(n) + kUrWarps) * ur_n4(n) * 4;
+}
 
 // Bounded spin of thread 0 until *ctr >= target.  False on timeout or when an
 // error is already flagged.
@@ -179,6 +188,78 @@ KSVD_DEV void red_release_add(unsigned* p, unsigned v) {
   asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
+// A partial travels between CTAs as 16-byte words {three floats, tag}: each word is
+// one 128-bit access, so a reader that finds the tag of the step it waits for
+// has the three values with it.  No counter, fence or second read follows the
+// store (a release on a counter, its poll and the read of the partials took
+// two L2 round trips more per power step).
+__host__ __device__ inline int ur_words(int n) { return (ur_n4(n) + 2) / 3; }
+
+KSVD_DEV void st_word(uint4* p, float x, float y, float z, unsigned tag) {
+  const unsigned long long lo = (static_cast<unsigned long long>(__float_as_uint(y)) << 32) | __float_as_uint(x);
+  const unsigned long long hi = (static_cast<unsigned long long>(tag) << 32) | __float_as_uint(z);
+  asm volatile("{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], t;\n}" ::"l"(p), "l"(lo),
+               "l"(hi)
+               : "memory");
+}
+
+KSVD_DEV uint4 ld_word(const uint4* p) {
+  unsigned long long lo, hi;
+  asm volatile("{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}"
+               : "=l"(lo), "=l"(hi)
+               : "l"(p)
+               : "memory");
+  return make_uint4(unsigned(lo), unsigned(lo >> 32), unsigned(hi), unsigned(hi >> 32));
+}
+
+// Sum of the words p[0], p[stride], ... (count of them) in ascending order, once
+// they show the tag: up to kB are polled together (re-reading one word after the
+// other would cost an L2 round trip each).  w of the result: 1, or 0 when the
+// time is over or an error is flagged elsewhere.
+KSVD_DEV float4 ur_gather(const uint4* p, size_t stride, int count, unsigned tag, GridBarrier* flags) {
+  constexpr int kB = 8;
+  float4 a = make_float4(0.f, 0.f, 0.f, 1.f);
+  for (int i = 0; i < count; i += kB) {
+    uint4 v[kB];
+#pragma unroll
+    for (int k = 0; k < kB; ++k) v[k] = (i + k < count) ? ld_word(p + (i + k) * stride) : make_uint4(0u, 0u, 0u, tag);
+    unsigned spins = 0;
+    unsigned long long t0 = 0;
+    for (;;) {
+      bool ready = true;
+#pragma unroll
+      for (int k = 0; k < kB; ++k) ready = ready && v[k].w == tag;
+      if (ready) break;
+#pragma unroll
+      for (int k = 0; k < kB; ++k)
+        if (v[k].w != tag) v[k] = ld_word(p + (i + k) * stride);
+      if ((++spins & 63u) == 0u) {
+        const unsigned long long t = globaltimer_ns();
+        if (t0 == 0) t0 = t;
+        if (t - t0 > kBarrierTimeoutNs) atomicCAS(&flags->err, DEVERR_NONE, DEVERR_TIMEOUT);
+        if (ld_relaxed_i32(&flags->err) != DEVERR_NONE) {
+          a.w = 0.0f;
+          return a;
+        }
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kB; ++k) {
+      a.x += __uint_as_float(v[k].x);
+      a.y += __uint_as_float(v[k].y);
+      a.z += __uint_as_float(v[k].z);
+    }
+  }
+  return a;
+}
+
+// Phase timer of one thread: the time since the last mark goes to `slot`.
+__device__ __noinline__ void ur_lap(unsigned long long* ph, int slot) {
+  const unsigned long long t = globaltimer_ns();
+  ph[slot] += t - ph[8];
+  ph[8] = t;
+}
+
 // One launch sweeps one or several problems (images): group g owns the CTAs
 // [cta_begin, cta_begin + ctas) and walks its own atoms with its own buffers,
 // counters and partials.  Groups whose ranges share CTAs run one after the
@@ -186,234 +267,287 @@ KSVD_DEV void red_release_add(unsigned* p, unsigned v) {
 // own CTAs, and every CTA takes its groups in the same (table) order, so the
 // lowest unfinished group always has all its CTAs and the launch cannot
 // deadlock.
+//
+// What bounds the sweep is the latency of K atoms in sequence, each a handful
+// of dependent steps (128 x 128 image, 8 x 8 patches, 256 atoms: 10 us an atom,
+// 14.5 with one thread per column, warp 0 finishing each step and a counter for
+// every exchange; 1000 x 777, 10 x 11 patches: 16 us, 25 before), so all that is not needed for the next step is kept off
+// them: the slices of the atoms are tabulated, an atom's entries, old
+// coefficients and old atom arrive during the atom before, e = r + x d_old is
+// formed inside the first pass over the columns, and every warp finishes a
+// power step for itself from the summed w.  The sums are in a fixed order
+// (dot_u, the column groups, the groups of partials), whatever thread makes them.
 template <int NW>
 __global__ void __launch_bounds__(kUrThreads, 1)
-    update_res_kernel(const UpdBatch batch, GridBarrier* flags, DevStats* stats, int timers) {
+    update_res_kernel(const __grid_constant__ UpdBatch batch, GridBarrier* flags, DevStats* stats, int timers) {
   extern __shared__ __align__(16) unsigned char ursm[];
   __shared__ int s_ok;
-  __shared__ int s_stop;
   __shared__ __align__(8) unsigned long long s_mbar;  // completion of the residual-row bulk copies
-  __shared__ unsigned long long s_ph[8];  // phase times of this CTA (slots 0..7)
+  __shared__ unsigned long long s_ph[9];  // phase times of this CTA (slots 0..7), the last mark
+  constexpr int KF = (NW + 3) / 4;        // float4 per lane of a row of up to 32 NW features
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   unsigned mpar = 0;  // parity of the next phase of s_mbar
   if (tid == 0) {
     mbar_init(&s_mbar, 1);
     fence_mbar_init();
   }
-  __syncthreads();
 
   // phase times gather in shared memory and are flushed once at the end
   const bool timer = (timers != 0 && blockIdx.x == 0 && tid == 0);
   if (timer)
     for (int k = 0; k < 8; ++k) s_ph[k] = 0ull;
-  unsigned long long tmark = timer ? globaltimer_ns() : 0ull;
+  if (timer) s_ph[8] = globaltimer_ns();
   auto lap = [&](int slot) {
-    if (timer) {
-      const unsigned long long t = globaltimer_ns();
-      s_ph[slot] += t - tmark;
-      tmark = t;
-    }
-  };
-  // thread 0 waits, the block learns the outcome
-  auto block_wait = [&](const unsigned* ctr, unsigned target) -> bool {
-    if (tid == 0) s_ok = ur_wait_count(ctr, target, flags) ? 1 : 0;
-    __syncthreads();
-    const bool ok = s_ok != 0;
-    __syncthreads();
-    return ok;
+    if (timer) ur_lap(s_ph, slot);
   };
 
   // every group whose CTA range holds this CTA, in the order of the table
   for (int gi = 0; gi < batch.ngroups; ++gi) {
     const UpdGroup& grp = batch.g[gi];
     if (int(blockIdx.x) < grp.cta_begin || int(blockIdx.x) >= grp.cta_begin + grp.ctas) continue;
-    __syncthreads();  // the previous group's shared memory is no longer read
     float* const R = grp.R;
     float* const D = grp.D;
     float* const coef = grp.coef;
-    const int* __restrict__ const atom_ptr = grp.atom_ptr;
     const int* __restrict__ const entries = grp.entries;
     const int* __restrict__ const last = grp.last;
-    float* const gw = grp.gw;
-    unsigned* const sync = grp.sync;
     const int n = grp.n, K = grp.K, L = grp.L, q1_cap = grp.q1_cap, cap = grp.cap;
     const int slice_target = grp.slice_target > 0 ? grp.slice_target : kUrDefaultSlice;
-    const int n4 = ur_n4(n), es = ur_es(n);
+    const int n4 = ur_n4(n), es = ur_es(n), W = ur_words(n), Gr = ur_groups(n);
     const int F = n4 / 4, es4 = es / 4;  // float4 per row of u / w, per resident column
-    float* Es = reinterpret_cast<float*>(ursm);
-    const float4* Es4 = reinterpret_cast<const float4*>(ursm);
-    int* ent_b = reinterpret_cast<int*>(ursm + size_t(cap) * es * 4);  // [2][cap]
-    float* xold_b = reinterpret_cast<float*>(ent_b + 2 * cap);           // [2][cap]
-    int* keep_b = reinterpret_cast<int*>(xold_b + 2 * cap);  // [2][cap]: residual row stored back
-    float* u = reinterpret_cast<float*>(keep_b + 2 * cap);
-    float* dold = u + n4;
-    float* dnext = dold + n4;
-    float* wred = dnext + n4;  // [kUrRows][n4]
-    float4* u4 = reinterpret_cast<float4*>(u);
-    const float4* dold4 = reinterpret_cast<const float4*>(dold);
-    float4* wred4 = reinterpret_cast<float4*>(wred);
-
     const int G = grp.ctas, b = int(blockIdx.x) - grp.cta_begin;
-    unsigned* iter_cnt = sync;
-    unsigned* done_cnt = sync + K;
-    int Gr = kUrThreads / F;  // column groups of the w pass, partial groups of the all-reduce
-    if (Gr > 16) Gr = 16;
-    if (Gr < 1) Gr = 1;
+    uint4* const words = static_cast<uint4*>(grp.gw);  // [2][G][W] partials, by parity of the step
+    unsigned* const done_cnt = reinterpret_cast<unsigned*>(words + size_t(2) * G * W);
+    unsigned* const iter_cnt = done_cnt + K;
+    float* const raw = reinterpret_cast<float*>(words + size_t(2) * G * W + (K + 1) / 2);  // [2][G][n4] plain partials
+    float* const Es = reinterpret_cast<float*>(ursm);
+    float4* const Es4 = reinterpret_cast<float4*>(ursm);
+    int* const row_b = reinterpret_cast<int*>(ursm + size_t(cap) * es * 4);  // [2][cap] patches
+    float* const xold_b = reinterpret_cast<float*>(row_b + 2 * cap);         // [2][cap]
+    int4* const tab = reinterpret_cast<int4*>(xold_b + 2 * cap);
+    float* const ut = reinterpret_cast<float*>(tab + kUrTab);  // [4][ft] ut[c][f] = u[4 f + c]
+    const int ft = ur_ft(n);
+    float* const u = ut + 4 * ft;
+    float* const dbuf = u + n4;        // [2][n4] old atom: this one's and the next one's
+    float* const wsum = dbuf + 2 * n4;
+    float* const wred = wsum + n4;     // [Gr][n4] sums over column groups, over groups of partials
+    float* const wstr = wred + Gr * n4;  // [16][n4] sums over the streamed columns of a warp
+    float* const xrow = wstr;            // [Gr][n4] sums over groups of partials
+    const int x_g = tid / W, x_f = tid - x_g * W;  // this thread's first group and word
+    const int s_q = tid / F, s_f = tid - s_q * F;  // its first column and float4 of the row stores, the stride
+    const int d_q = kUrThreads / F, d_f = kUrThreads - d_q * F;
+    float4* const u4 = reinterpret_cast<float4*>(u);
+    const float4* const wsum4 = reinterpret_cast<const float4*>(wsum);
     // bulk copies need 16-byte aligned rows of a multiple of 16 bytes
     const bool tma = (n & 3) == 0 && (reinterpret_cast<uintptr_t>(R) & 15) == 0;
+    // w pass: the warp's column group and its share of the 32-feature chunks
+    const int H = kUrWarps / Gr, wg = warp % Gr, wh = warp / Gr;
 
-    // this CTA's slice [sb, se) of atom a's c entries starting at beg
-    auto slice_of = [&](int a, int& beg, int& c, int& active, int& sb, int& se) {
-      beg = atom_ptr[a];
-      c = atom_ptr[a + 1] - beg;
-      active = ur_active(c, G, slice_target);
-      sb = int(int64_t(c) * b / active);
-      se = int(int64_t(c) * (b + 1) / active);
+    // this CTA's slice [sb, sb + m) of each of the next kUrTab atoms' c entries:
+    // first entry, m (-1: no part in the atom), entries that enter the power
+    // iteration, CTAs on the atom (0: unused atom)
+    auto fill_tab = [&](int a0) {
+      __syncthreads();
+      for (int t = tid; t < kUrTab && a0 + t < K; t += kUrThreads) {
+        const int beg = __ldg(grp.atom_ptr + a0 + t), c = __ldg(grp.atom_ptr + a0 + t + 1) - beg;
+        const int active = c > 0 ? ur_active(c, G, slice_target) : 0;
+        int sb = 0, m = -1, mc = 0;
+        if (b < active) {
+          sb = int(int64_t(c) * b / active);
+          m = int(int64_t(c) * (b + 1) / active) - sb;
+          const int c_eff = (q1_cap && c > 1024) ? 1024 : c;
+          mc = max(0, min(m, c_eff - sb));
+        }
+        tab[t] = make_int4(beg + sb, m, mc, active);
+      }
+      __syncthreads();
     };
-    // entries, old coefficients and store-back flags of [sb, sb + cnt) into
-    // meta buffer `slot` and atom a into dst (all threads; several loads in
-    // flight per thread).  A residual row is stored back unless a is the last
+    // patches and old coefficients of the first `cnt` columns of a slice into meta
+    // buffer `slot`, in three steps (thread t: column t, so the loads of one step
+    // may be in flight while the block does something else).  A patch's
+    // complement marks a residual row that is not stored back: a is the last
     // atom of the patch's support.
-    auto load_meta = [&](int beg, int sb, int cnt, int slot, int a, float* dst) {
-      int* ent = ent_b + slot * cap;
-      float* xo = xold_b + slot * cap;
-      int* kp = keep_b + slot * cap;
-      constexpr int kB = 4;
-      for (int t0 = tid; t0 < cnt; t0 += kUrThreads * kB) {
-        int e[kB];
-#pragma unroll
-        for (int k = 0; k < kB; ++k) {
-          const int t = t0 + k * kUrThreads;
-          e[k] = (t < cnt) ? __ldg(entries + beg + sb + t) : 0;
-        }
-        float x[kB];
-        int lt[kB];
-#pragma unroll
-        for (int k = 0; k < kB; ++k) {
-          const bool in = t0 + k * kUrThreads < cnt;
-          x[k] = in ? __ldcg(coef + e[k]) : 0.0f;
-          lt[k] = (in && last != nullptr) ? __ldg(last + e[k] / L) : -1;
-        }
-#pragma unroll
-        for (int k = 0; k < kB; ++k) {
-          const int t = t0 + k * kUrThreads;
-          if (t < cnt) {
-            ent[t] = e[k];
-            xo[t] = x[k];
-            kp[t] = (lt[k] != a) ? 1 : 0;
+    struct Meta {
+      int en, pt, lt;
+      float x;
+    };
+    auto meta_entry = [&](Meta& md, int first, int cnt, int t) {
+      md.en = t < cnt ? __ldg(entries + first + t) : -1;
+    };
+    auto meta_rest = [&](Meta& md) {
+      md.x = md.en >= 0 ? __ldcg(coef + md.en) : 0.0f;
+      md.pt = md.en >= 0 ? md.en / L : 0;
+      md.lt = (md.en >= 0 && last != nullptr) ? __ldg(last + md.pt) : -1;
+    };
+    auto meta_store = [&](const Meta& md, int slot, int a, int t) {
+      if (md.en >= 0) {
+        row_b[slot * cap + t] = md.lt != a ? md.pt : ~md.pt;
+        xold_b[slot * cap + t] = md.x;
+      }
+    };
+    auto row_of = [](int p) -> int64_t { return p >= 0 ? p : ~p; };
+    // u . e_q for a resident column: four chains, chain c over the features
+    // 4 f + c, one per lane of four; (a0 + a1) + (a2 + a3) in every lane.  With
+    // `form`, e = r + x d is formed in place first.  The four lanes' words of a
+    // column and the eight columns of a warp sit in distinct banks, and u comes
+    // four features of a chain at a time from its transposed copy.
+    auto dot_u = [&](int q, bool in, bool form, float x) -> float {
+      float* const er = Es + size_t(q) * es + (lane & 3);
+      const float4* const uc = reinterpret_cast<const float4*>(ut + (lane & 3) * ft);
+      float a = 0.0f;
+      if (in) {
+        auto term = [&](int f, float w) {
+          float e = er[4 * f];
+          if (form) {
+            e = fmaf(x, w, e);
+            er[4 * f] = e;
           }
+          a = fmaf(e, w, a);
+        };
+        int f = 0;
+#pragma unroll 2
+        for (; f + 4 <= F; f += 4) {
+          const float4 w = uc[f >> 2];
+          float e0 = er[4 * f], e1 = er[4 * f + 4], e2 = er[4 * f + 8], e3 = er[4 * f + 12];
+          if (form) {
+            e0 = fmaf(x, w.x, e0);
+            e1 = fmaf(x, w.y, e1);
+            e2 = fmaf(x, w.z, e2);
+            e3 = fmaf(x, w.w, e3);
+            er[4 * f] = e0;
+            er[4 * f + 4] = e1;
+            er[4 * f + 8] = e2;
+            er[4 * f + 12] = e3;
+          }
+          a = fmaf(e0, w.x, a);
+          a = fmaf(e1, w.y, a);
+          a = fmaf(e2, w.z, a);
+          a = fmaf(e3, w.w, a);
         }
+        for (; f < F; ++f) term(f, ut[(lane & 3) * ft + f]);
       }
-      for (int i = tid; i < n4; i += kUrThreads) dst[i] = (i < n) ? __ldcg(D + int64_t(a) * n + i) : 0.0f;
+      a += __shfl_xor_sync(0xffffffffu, a, 1);
+      a += __shfl_xor_sync(0xffffffffu, a, 2);
+      return a;
     };
-    // u . e_q for a resident column (one thread, 16-byte loads, 4 chains)
-    auto dot_u = [&](int q) -> float {
-      const float4* er = Es4 + size_t(q) * es4;
-      float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-#pragma unroll 6
-      for (int f = 0; f < F; ++f) {
-        const float4 e = er[f], w = u4[f];
-        a0 = fmaf(e.x, w.x, a0);
-        a1 = fmaf(e.y, w.y, a1);
-        a2 = fmaf(e.z, w.z, a2);
-        a3 = fmaf(e.w, w.w, a3);
-      }
-      return (a0 + a1) + (a2 + a3);
-    };
+    const int q_l = warp * 8 + (lane >> 2);  // this lane's column of 128
 
     int jprev = -1, aprev = 0;
-    int slot = 0;        // meta buffer of the current atom
-    int meta_atom = -1;  // atom whose meta was prefetched into buffer `slot`
+    int slot = 0;        // meta and old-atom buffer of the current atom
+    int meta_atom = -1;  // atom whose meta is in buffer `slot`
     for (int j = 0; j < K; ++j) {
-      int beg, c, active, sb, se;
-      slice_of(j, beg, c, active, sb, se);
-      if (c == 0) continue;
+      if (j % kUrTab == 0) fill_tab(j);
+      const int4 sl = tab[j % kUrTab];
+      const int first = sl.x, m = sl.y, mc = sl.z, active = sl.w;
+      if (active == 0) continue;
       const int jp = jprev, ap = aprev;
       jprev = j;
       aprev = active;
-      if (b >= active) continue;
-      const int c_eff = (q1_cap && c > 1024) ? 1024 : c;
-      const int m = se - sb;
-      const int mres = m < cap ? m : cap;
-      // columns [0, mc) of the slice enter the power iteration
-      int mc = c_eff - sb;
-      mc = mc < 0 ? 0 : (mc > m ? m : mc);
-      const int mcr = mc < cap ? mc : cap;  // of which resident
-      const bool streamed = mc > cap;        // some enter from the residual
-      const int* ent_s = ent_b + slot * cap;
-      const float* xold_s = xold_b + slot * cap;
-      float* v_s = xold_b + slot * cap;  // per-column scalars once the columns are built
-      const int* keep_s = keep_b + slot * cap;
+      if (m < 0) continue;
+      const int mres = min(m, cap);
+      const int mcr = min(mc, cap);   // resident columns in the power iteration
+      const bool streamed = mc > cap;  // some enter from the residual
+      const bool alone = active == 1;
+      // Partials of many CTAs: as plain rows behind a counter, which one thread
+      // polls, instead of as tagged words that every thread polls.  Tagged words
+      // save a release and a round trip a step (1.8 against 2.1 us with 9 CTAs,
+      // 144 features), but each carries a quarter more bytes and the polls of many
+      // CTAs slow the stores they wait for (3.2 against 3.0 us with 141 CTAs).
+      const bool counted = active > 2 * Gr;
+      float* const v_s = xold_b + slot * cap;  // old coefficients, then per-column scalars
+      const int* const row_s = row_b + slot * cap;
+      const float* const dold = dbuf + slot * n4;
+      const float4* const dold4 = reinterpret_cast<const float4*>(dold);
 
       // ---- entries, old coefficients and the old atom: never written by other
-      // atoms, so read before the wait (or prefetched during the previous atom)
-      if (meta_atom == j) {
-        for (int i = tid; i < n4; i += kUrThreads) dold[i] = dnext[i];
-      } else {
-        load_meta(beg, sb, mres, slot, j, dold);
+      // atoms, so read before the wait (or during the previous atom)
+      if (meta_atom != j) {
+        for (int t = tid; t < mres; t += kUrThreads) {
+          Meta md;
+          meta_entry(md, first, mres, t);
+          meta_rest(md);
+          meta_store(md, slot, j, t);
+        }
+        for (int i = tid; i < n4; i += kUrThreads) {
+          const float d = (i < n) ? __ldcg(D + int64_t(j) * n + i) : 0.0f;
+          dbuf[slot * n4 + i] = d;
+          ut[(i & 3) * ft + (i >> 2)] = d;
+        }
+        __syncthreads();
       }
       lap(7);
-      __syncthreads();
-      if (jp >= 0 && !block_wait(done_cnt + jp, unsigned(ap))) return;
+      // the previous atom's residual rows (what this CTA stored alone needs no wait)
+      if (jp >= 0 && (ap > 1 || b > 0)) {
+        if (tid == 0) s_ok = ur_wait_count(done_cnt + jp, unsigned(ap), flags) ? 1 : 0;
+        __syncthreads();
+        if (!s_ok) return;
+      }
       lap(0);
 
-      // the next non-empty atom; if this CTA works on it, its meta is fetched
-      // while this CTA waits for the first partials
-      int jn = j + 1;
-      while (jn < K && atom_ptr[jn + 1] == atom_ptr[jn]) ++jn;
-      int nbeg = 0, nc = 0, nact = 0, nsb = 0, nse = 0;
-      bool prefetch = false;
-      if (jn < K) {
-        slice_of(jn, nbeg, nc, nact, nsb, nse);
-        prefetch = b < nact;
-      }
-
-      // ---- resident columns e_q = r_q + x_q d_old ---------------------------
+      // ---- residual rows ----------------------------------------------------
+      bool ok = true;
       if (tma) {
-        // residual rows by bulk copies (the residual was written by other CTAs
-        // through the generic proxy: acquire above, proxy fence here), then
-        // e = r + x d in place
+        // bulk copies (the residual was written by other CTAs through the generic
+        // proxy: acquire above, proxy fence here)
         if (tid == 0) mbar_arrive_expect_tx(&s_mbar, unsigned(mres) * unsigned(n) * 4u);
-        __syncthreads();
         asm volatile("fence.proxy.async.global;" ::: "memory");
         for (int q = tid; q < mres; q += kUrThreads)
-          bulk_g2s(Es + size_t(q) * es, R + int64_t(ent_s[q] / L) * n, unsigned(n) * 4u, &s_mbar);
-        const bool ok = mbar_wait(&s_mbar, mpar, kBarrierTimeoutNs);
-        mpar ^= 1u;
-        if (__syncthreads_or(!ok)) {
-          if (tid == 0) atomicCAS(&flags->err, DEVERR_NONE, DEVERR_TIMEOUT);
-          return;
-        }
-        for (int t = tid; t < mres * F; t += kUrThreads) {
-          const int q = t / F, f = t - q * F;
-          const float x = xold_s[q];
-          const float4 d = dold4[f];
-          float4* ep = reinterpret_cast<float4*>(Es) + size_t(q) * es4 + f;
-          float4 e = *ep;
-          e.x = fmaf(x, d.x, e.x);
-          e.y = fmaf(x, d.y, e.y);
-          e.z = fmaf(x, d.z, e.z);
-          e.w = fmaf(x, d.w, e.w);
-          *ep = e;
-        }
+          bulk_g2s(Es + size_t(q) * es, R + row_of(row_s[q]) * n, unsigned(n) * 4u, &s_mbar);
       } else {
-        for (int t = tid; t < mres * n4; t += kUrThreads) {
-          const int q = t / n4, i = t - q * n4;
-          float e = 0.0f;
-          if (i < n) e = fmaf(xold_s[q], dold[i], __ldcg(R + int64_t(ent_s[q] / L) * n + i));
-          Es[size_t(q) * es + i] = e;
+        for (int q = warp; q < mres; q += 2 * kUrWarps) {
+          const int q1 = q + kUrWarps;
+          const float* ra = R + row_of(row_s[q]) * n;
+          const float* rb = R + (q1 < mres ? row_of(row_s[q1]) : 0) * n;
+          float r0[NW], r1[NW];
+#pragma unroll
+          for (int k = 0; k < NW; ++k) {
+            const int i = lane + 32 * k;
+            r0[k] = i < n ? __ldcg(ra + i) : 0.0f;
+            r1[k] = i < n && q1 < mres ? __ldcg(rb + i) : 0.0f;
+          }
+#pragma unroll
+          for (int k = 0; k < NW; ++k) {
+            const int i = lane + 32 * k;
+            if (i < n4) Es[size_t(q) * es + i] = r0[k];
+            if (i < n4 && q1 < mres) Es[size_t(q1) * es + i] = r1[k];
+          }
         }
       }
-      for (int i = tid; i < n4; i += kUrThreads) u[i] = dold[i];
-      __syncthreads();
+
+      // the entry of this thread's column, for its new coefficient
+      const int c_en = (lane & 3) == 0 && q_l < mres ? __ldg(entries + first + q_l) : 0;
+
+      // the next non-empty atom; if this CTA works on it, its meta is fetched
+      // while this one is worked on
+      int jn = j + 1;
+      while (jn < K && jn % kUrTab != 0 && tab[jn % kUrTab].w == 0) ++jn;
+      int nact = 2;  // its CTAs (beyond the table: assume several)
+      bool prefetch = false;
+      Meta nm{-1, 0, -1, 0.0f};
+      float nd = 0.0f;
+      if (jn < K && jn % kUrTab != 0) {
+        const int4 ns = tab[jn % kUrTab];
+        nact = ns.w;
+        prefetch = ns.y >= 0 && ns.y <= kUrThreads;
+        if (prefetch) {
+          meta_entry(nm, ns.x, min(ns.y, cap), tid);
+          nd = (tid < n) ? __ldcg(D + int64_t(jn) * n + tid) : 0.0f;
+        }
+      }
       lap(1);
+      if (tma) {
+        ok = mbar_wait(&s_mbar, mpar, kBarrierTimeoutNs);
+        mpar ^= 1u;
+        if (!ok) atomicCAS(&flags->err, DEVERR_NONE, DEVERR_TIMEOUT);  // the block returns after the next step's sum
+      } else {
+        __syncthreads();
+      }
 
       // Two streamed columns (q0, q1 = q0 + kUrWarps, both >= cap) from the
       // residual; a column index >= lim gives zeros.
       auto stream_cols = [&](int q0, int lim, float (&e0)[NW], float (&e1)[NW], int& ea, int& eb) {
         const int q1 = q0 + kUrWarps;
-        ea = (q0 < lim) ? __ldg(entries + beg + sb + q0) : -1;
-        eb = (q1 < lim) ? __ldg(entries + beg + sb + q1) : -1;
+        ea = (q0 < lim) ? __ldg(entries + first + q0) : -1;
+        eb = (q1 < lim) ? __ldg(entries + first + q1) : -1;
         const float xa = (ea >= 0) ? __ldcg(coef + ea) : 0.0f;
         const float xb = (eb >= 0) ? __ldcg(coef + eb) : 0.0f;
         const float* ra = R + int64_t(ea >= 0 ? ea / L : 0) * n;
@@ -427,17 +561,35 @@ __global__ void __launch_bounds__(kUrThreads, 1)
       };
 
       // ---- power iteration ---------------------------------------------------
+      float4 uo[KF];  // u in the registers of every warp: float4 lane + 32 k
+#pragma unroll
+      for (int k = 0; k < KF; ++k)
+        uo[k] = (lane + 32 * k < F) ? dold4[lane + 32 * k] : make_float4(0.f, 0.f, 0.f, 0.f);
       int iters = 0;
-      float dprev = 0.0f;  // warp 0: the previous step's change
+      float dprev = 0.0f;  // the previous step's change
       for (int it = 0; it < kUrMaxIters; ++it) {
-        // v_q = u . e_q, one thread per resident column
-        for (int q = tid; q < mcr; q += kUrThreads) v_s[q] = dot_u(q);
+        // v_q = u . e_q (u is d_old in the first step)
+        const float* const uc = it == 0 ? dold : u;
+        if (it == 0) {
+          for (int q0 = 0; q0 + warp * 8 < mres; q0 += kUrThreads / 4) {
+            const int q = q0 + q_l;
+            const bool in = q < mres;
+            const float v = dot_u(q, in, true, in ? v_s[q] : 0.0f);
+            if (in && (lane & 3) == 0) v_s[q] = v;
+          }
+        } else {
+          for (int q0 = 0; q0 + warp * 8 < mcr; q0 += kUrThreads / 4) {
+            const int q = q0 + q_l;
+            const float v = dot_u(q, q < mcr, false, 0.0f);
+            if (q < mcr && (lane & 3) == 0) v_s[q] = v;
+          }
+        }
         if (streamed) {  // columns beyond the capacity: a warp per two columns
           float ur[NW], wacc[NW];
 #pragma unroll
           for (int k = 0; k < NW; ++k) {
             const int i = lane + 32 * k;
-            ur[k] = (i < n) ? u[i] : 0.0f;
+            ur[k] = (i < n) ? uc[i] : 0.0f;
             wacc[k] = 0.0f;
           }
           for (int q = cap + warp; q < mc; q += 2 * kUrWarps) {
@@ -461,65 +613,92 @@ __global__ void __launch_bounds__(kUrThreads, 1)
 #pragma unroll
           for (int k = 0; k < NW; ++k) {
             const int i = lane + 32 * k;
-            if (i < n4) wred[(16 + warp) * n4 + i] = wacc[k];
+            if (i < n4) wstr[warp * n4 + i] = wacc[k];
           }
         }
         __syncthreads();
-        // w = sum_q v_q e_q: column group g (q = g mod Gr) of float4 column f
-        {
-          const int f = tid % F, g = tid / F;
-          if (g < Gr) {
-            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-            for (int q = g; q < mcr; q += Gr) {
-              const float v = v_s[q];
-              const float4 e = Es4[size_t(q) * es4 + f];
-              acc.x = fmaf(v, e.x, acc.x);
-              acc.y = fmaf(v, e.y, acc.y);
-              acc.z = fmaf(v, e.z, acc.z);
-              acc.w = fmaf(v, e.w, acc.w);
-            }
-            wred4[g * F + f] = acc;
-          }
-        }
-        __syncthreads();
-        float4* gwp = reinterpret_cast<float4*>(gw + (size_t(it & 1) * G + b) * n4);
-        for (int f = tid; f < F; f += kUrThreads) {
-          float4 acc = wred4[f];
-#pragma unroll 4
-          for (int g = 1; g < Gr; ++g) {
-            const float4 v = wred4[g * F + f];
-            acc.x += v.x;
-            acc.y += v.y;
-            acc.z += v.z;
-            acc.w += v.w;
-          }
-          if (streamed)
+        // w = sum_q v_q e_q: the columns q = wg, wg + Gr, ... of a group, lanes
+        // over the features, the 32-feature chunks wh, wh + H, ...
+        if (H == 1) {
+          if (warp < Gr) {
+            float acc[NW];
 #pragma unroll
-            for (int w = 0; w < kUrWarps; ++w) {
-              const float4 v = wred4[(16 + w) * F + f];
-              acc.x += v.x;
-              acc.y += v.y;
-              acc.z += v.z;
-              acc.w += v.w;
+            for (int k = 0; k < NW; ++k) acc[k] = 0.0f;
+#pragma unroll 2
+            for (int q = warp; q < mcr; q += Gr) {
+              const float v = v_s[q];
+              const float* const eq = Es + size_t(q) * es + lane;
+#pragma unroll
+              for (int k = 0; k < NW; ++k)
+                if (32 * k + lane < n4) acc[k] = fmaf(v, eq[32 * k], acc[k]);
             }
-          __stcg(gwp + f, acc);
+#pragma unroll
+            for (int k = 0; k < NW; ++k)
+              if (32 * k + lane < n4) wred[warp * n4 + 32 * k + lane] = acc[k];
+          }
+        } else if (wh < H) {
+          constexpr int kC = 6;  // chunks of a warp (H grows as Gr falls)
+          float acc[kC];
+#pragma unroll
+          for (int k = 0; k < kC; ++k) acc[k] = 0.0f;
+#pragma unroll 2
+          for (int q = wg; q < mcr; q += Gr) {
+            const float v = v_s[q];
+            const float* const eq = Es + size_t(q) * es + 32 * wh + lane;
+#pragma unroll
+            for (int k = 0; k < kC; ++k)
+              if (32 * (wh + H * k) + lane < n4) acc[k] = fmaf(v, eq[32 * H * k], acc[k]);
+          }
+#pragma unroll
+          for (int k = 0; k < kC; ++k)
+            if (32 * (wh + H * k) + lane < n4) wred[wg * n4 + 32 * (wh + H * k) + lane] = acc[k];
         }
         __syncthreads();
         lap(2);
-        if (tid == 0) red_release_add(iter_cnt + j, 1u);
-        if (it == 0 && prefetch)  // overlaps the wait below
-          load_meta(nbeg, nsb, min(nse - nsb, cap), slot ^ 1, jn, dnext);
-        if (!block_wait(iter_cnt + j, unsigned(it + 1) * unsigned(active))) return;
-        lap(3);
-        // all-reduce: group g sums partials g, g + Gr, ... of float4 column f in
-        // ascending order (loads batched)
+        // the CTA's w, an element per thread; with several CTAs three elements
+        // are packed into a word by the first of their threads
+        const unsigned tag = (unsigned(j) << 8) + unsigned(it) + 1u;
         {
-          const int f = tid % F, g = tid / F;
+          uint4* const wp = words + (size_t(it & 1) * G + b) * W;
+          for (int i0 = warp * 30; i0 < 3 * W; i0 += kUrWarps * 30) {
+            const int i = i0 + lane;
+            float s = 0.0f;
+            if (lane < 30 && i < n4) {
+              s = wred[i];
+#pragma unroll 8
+              for (int g = 1; g < Gr; ++g) s += wred[g * n4 + i];
+              if (streamed)
+#pragma unroll
+                for (int w = 0; w < kUrWarps; ++w) s += wstr[w * n4 + i];
+            }
+            if (alone) {
+              if (lane < 30 && i < n4) wsum[i] = s;
+            } else {
+              const float y = __shfl_down_sync(0xffffffffu, s, 1), z = __shfl_down_sync(0xffffffffu, s, 2);
+              if (counted) {
+                if (lane < 30 && i < n4) __stcg(raw + (size_t(it & 1) * G + b) * n4 + i, s);
+              } else if (lane < 30 && lane % 3 == 0 && i / 3 < W) {
+                st_word(wp + i / 3, s, y, z, tag);
+              }
+            }
+          }
+        }
+        if (counted) {
+          __syncthreads();
+          if (tid == 0) red_release_add(iter_cnt + j, 1u);
+        }
+        if (it == 0 && prefetch) meta_rest(nm);
+        if (counted) {
+          // group g sums rows g, g + Gr, ... of float4 column f
+          if (tid == 0) s_ok = ur_wait_count(iter_cnt + j, unsigned(it + 1) * unsigned(active), flags) ? 1 : 0;
+          __syncthreads();
+          if (!s_ok) return;
+          const int g = s_q, f = s_f;
           if (g < Gr) {
             float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-            const float4* base = reinterpret_cast<const float4*>(gw + size_t(it & 1) * G * n4) + f;
-            constexpr int kB = 12;  // one round of loads for up to 12 Gr partials per thread
+            const float4* const base = reinterpret_cast<const float4*>(raw + size_t(it & 1) * G * n4) + f;
+            constexpr int kB = 11;  // loads in flight
+#pragma unroll 1
             for (int bb0 = g; bb0 < active; bb0 += Gr * kB) {
               float4 v[kB];
 #pragma unroll
@@ -535,93 +714,119 @@ __global__ void __launch_bounds__(kUrThreads, 1)
                 acc.w += v[k].w;
               }
             }
-            wred4[g * F + f] = acc;
+            reinterpret_cast<float4*>(wred)[g * F + f] = acc;
           }
-        }
-        __syncthreads();
-        iters = it + 1;
-        // warp 0 finishes the step: w, its norm, the new u, the change, the
-        // stop decision and, when stopping, the sign (u . d_old >= 0)
-        if (warp == 0) {
-          constexpr int kF = 4;  // float4 per lane (F <= 128)
-          float4 wv[kF];
-          float s2 = 0.0f;
-#pragma unroll
-          for (int k = 0; k < kF; ++k) {
-            const int f = lane + 32 * k;
-            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (f < F)
+          __syncthreads();
+          if (tid < n4) {
+            float s = wred[tid];
 #pragma unroll 4
-              for (int g = 0; g < Gr; ++g) {
-                const float4 v = wred4[g * F + f];
-                acc.x += v.x;
-                acc.y += v.y;
-                acc.z += v.z;
-                acc.w += v.w;
-              }
-            wv[k] = acc;
-            s2 = fmaf(acc.x, acc.x, fmaf(acc.y, acc.y, fmaf(acc.z, acc.z, fmaf(acc.w, acc.w, s2))));
+            for (int g2 = 1; g2 < Gr; ++g2) s += wred[g2 * n4 + tid];
+            wsum[tid] = s;
           }
-          const float nrm2 = warp_sum(s2);
-          bool stop;
-          if (!(nrm2 > 0.0f)) {
-            stop = true;  // E == 0: keep the old atom direction
-          } else {
-            const float inv = 1.0f / sqrtf(nrm2);
-            float dm = 0.0f;
-#pragma unroll
-            for (int k = 0; k < kF; ++k) {
-              const int f = lane + 32 * k;
-              if (f < F) {
-                const float4 o = u4[f];
-                float4 un;
-                un.x = wv[k].x * inv;
-                un.y = wv[k].y * inv;
-                un.z = wv[k].z * inv;
-                un.w = wv[k].w * inv;
-                dm = fmaxf(dm, fmaxf(fmaxf(fabsf(un.x - o.x), fabsf(un.y - o.y)),
-                                     fmaxf(fabsf(un.z - o.z), fabsf(un.w - o.w))));
-                u4[f] = un;
-              }
+        } else if (!alone) {
+          // all-reduce: group g sums partials g, g + Gr, ... in ascending order,
+          // a word per thread; its rows go where the streamed columns' were
+          if (streamed) __syncthreads();
+          const int gs = min(Gr, active);
+          int g = x_g, f = x_f;
+#pragma unroll 1
+          while (g < gs) {
+            const float4 a = ur_gather(words + (size_t(it & 1) * G + g) * W + f, size_t(Gr) * W,
+                                       (active - g + Gr - 1) / Gr, tag, flags);
+            ok = ok && a.w != 0.0f;
+            float* const xr = xrow + g * n4 + 3 * f;
+            xr[0] = a.x;
+            if (3 * f + 1 < n4) xr[1] = a.y;
+            if (3 * f + 2 < n4) xr[2] = a.z;
+            f += kUrThreads;
+            while (f >= W) {
+              f -= W;
+              ++g;
             }
-            dm = warp_max(dm);
-            // stop when the change is below the tolerance, or when the observed
-            // contraction rho = dm / dprev puts the remaining distance to the
-            // limit, about dm rho / (1 - rho), below it
-            const float rho = (it > 0 && dprev > 0.0f) ? dm / dprev : 1.0f;
-            stop = dm < kUrTol || (rho < 0.5f && dm < 1e-3f && dm * rho < kUrTol * (1.0f - rho));
-            dprev = dm;
           }
-          if (stop) {
-            float sd = 0.0f;
-#pragma unroll
-            for (int k = 0; k < kF; ++k) {
-              const int f = lane + 32 * k;
-              if (f < F) {
-                const float4 a = u4[f], d = dold4[f];
-                sd = fmaf(a.x, d.x, fmaf(a.y, d.y, fmaf(a.z, d.z, fmaf(a.w, d.w, sd))));
-              }
-            }
-            sd = warp_sum(sd);
-            if (sd < 0.0f)
-#pragma unroll
-              for (int k = 0; k < kF; ++k) {
-                const int f = lane + 32 * k;
-                if (f < F) {
-                  float4 a = u4[f];
-                  a.x = -a.x;
-                  a.y = -a.y;
-                  a.z = -a.z;
-                  a.w = -a.w;
-                  u4[f] = a;
-                }
-              }
+          __syncthreads();
+          if (tid < n4) {
+            float s = xrow[tid];
+#pragma unroll 4
+            for (int g = 1; g < gs; ++g) s += xrow[g * n4 + tid];
+            wsum[tid] = s;
           }
-          if (lane == 0) s_stop = stop ? 1 : 0;
         }
+        if (__syncthreads_or(!ok)) return;
+        lap(3);
+        iters = it + 1;
+        // every warp finishes the step: w, its norm, the new u, the change, the
+        // stop decision (the same values in every warp of every CTA) and, when
+        // stopping, the sign (u . d_old >= 0)
+        float4 wv[KF];
+        float s2 = 0.0f;
+#pragma unroll
+        for (int k = 0; k < KF; ++k) {
+          const int f = lane + 32 * k;
+          const float4 acc = f < F ? wsum4[f] : make_float4(0.f, 0.f, 0.f, 0.f);
+          wv[k] = acc;
+          s2 = fmaf(acc.x, acc.x, fmaf(acc.y, acc.y, fmaf(acc.z, acc.z, fmaf(acc.w, acc.w, s2))));
+        }
+        const float nrm2 = warp_sum(s2);
+        bool stop;
+        if (!(nrm2 > 0.0f)) {
+          stop = true;  // E == 0: keep the old atom direction
+        } else {
+          const float inv = 1.0f / sqrtf(nrm2);
+          float dm = 0.0f;
+#pragma unroll
+          for (int k = 0; k < KF; ++k) {
+            const float4 o = uo[k];
+            float4 un;
+            un.x = wv[k].x * inv;
+            un.y = wv[k].y * inv;
+            un.z = wv[k].z * inv;
+            un.w = wv[k].w * inv;
+            dm = fmaxf(dm, fmaxf(fmaxf(fabsf(un.x - o.x), fabsf(un.y - o.y)),
+                                 fmaxf(fabsf(un.z - o.z), fabsf(un.w - o.w))));
+            uo[k] = un;
+          }
+          // never NaN nor negative (fmaxf), so its bits order as it does
+          dm = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(dm)));
+          // stop when the change is below the tolerance, or when the observed
+          // contraction rho = dm / dprev puts the remaining distance to the
+          // limit, about dm rho / (1 - rho), below it
+          stop = dm < kUrTol;
+          if (!stop && it > 0 && dprev > 0.0f && dm < 1e-3f) {
+            const float rho = dm / dprev;
+            stop = rho < 0.5f && dm * rho < kUrTol * (1.0f - rho);
+          }
+          dprev = dm;
+        }
+        if (stop) {
+          float sd = 0.0f;
+#pragma unroll
+          for (int k = 0; k < KF; ++k) {
+            const int f = lane + 32 * k;
+            if (f < F) {
+              const float4 a = uo[k], d = dold4[f];
+              sd = fmaf(a.x, d.x, fmaf(a.y, d.y, fmaf(a.z, d.z, fmaf(a.w, d.w, sd))));
+            }
+          }
+          sd = warp_sum(sd);
+          if (sd < 0.0f)
+#pragma unroll
+            for (int k = 0; k < KF; ++k) uo[k] = make_float4(-uo[k].x, -uo[k].y, -uo[k].z, -uo[k].w);
+        }
+        if (warp == 0)
+#pragma unroll
+          for (int k = 0; k < KF; ++k)
+            if (lane + 32 * k < F) {
+              const int f = lane + 32 * k;
+              u4[f] = uo[k];
+              ut[f] = uo[k].x;
+              ut[ft + f] = uo[k].y;
+              ut[2 * ft + f] = uo[k].z;
+              ut[3 * ft + f] = uo[k].w;
+            }
         __syncthreads();
         lap(4);
-        if (s_stop) break;
+        if (stop) break;
       }
       if (b == 0) {
         for (int i = tid; i < n; i += kUrThreads) __stcg(D + int64_t(j) * n + i, u[i]);
@@ -632,10 +837,13 @@ __global__ void __launch_bounds__(kUrThreads, 1)
       }
 
       // ---- coefficients x = u . e (0 beyond the cap) and residual e - x u ----
-      for (int q = tid; q < mres; q += kUrThreads) {
-        const float x = (q < mc) ? dot_u(q) : 0.0f;
-        v_s[q] = x;
-        __stcg(coef + ent_s[q], x);
+      for (int q0 = 0; q0 + warp * 8 < mres; q0 += kUrThreads / 4) {
+        const int q = q0 + q_l;
+        const float x = dot_u(q, q < mcr, false, 0.0f);
+        if (q < mres && (lane & 3) == 0) {
+          v_s[q] = q < mc ? x : 0.0f;
+          __stcg(coef + (q0 == 0 ? c_en : __ldg(entries + first + q)), q < mc ? x : 0.0f);
+        }
       }
       if (m > cap) {  // streamed columns: a warp per two columns
         float ur[NW];
@@ -683,36 +891,50 @@ __global__ void __launch_bounds__(kUrThreads, 1)
           }
         }
       }
+      if (prefetch) {  // the next atom's meta and old atom
+        meta_store(nm, slot ^ 1, jn, tid);
+        if (tid < n4) dbuf[(slot ^ 1) * n4 + tid] = nd;
+      }
       __syncthreads();
-      if (tma) {  // rows of 16-byte aligned float4
-        for (int t = tid; t < mres * F; t += kUrThreads) {
-          const int q = t / F, f = t - q * F;
-          if (!keep_s[q]) continue;
-          const float x = v_s[q];
-          const float4 e = Es4[size_t(q) * es4 + f], w = u4[f];
-          float4 r;
-          r.x = fmaf(-x, w.x, e.x);
-          r.y = fmaf(-x, w.y, e.y);
-          r.z = fmaf(-x, w.z, e.z);
-          r.w = fmaf(-x, w.w, e.w);
-          __stcg(reinterpret_cast<float4*>(R + int64_t(ent_s[q] / L) * n) + f, r);
+      if (prefetch && tid < n4) ut[(tid & 3) * ft + (tid >> 2)] = nd;
+      if (tma) {  // rows of 16-byte aligned float4, (row, float4) pairs over the threads
+        int q = s_q, f = s_f;
+#pragma unroll 2
+        while (q < mres) {
+          const int p = row_s[q];
+          if (p >= 0) {
+            const float x = v_s[q];
+            const float4 e = Es4[q * es4 + f], w = u4[f];
+            float4 r;
+            r.x = fmaf(-x, w.x, e.x);
+            r.y = fmaf(-x, w.y, e.y);
+            r.z = fmaf(-x, w.z, e.z);
+            r.w = fmaf(-x, w.w, e.w);
+            __stcg(reinterpret_cast<float4*>(R + int64_t(p) * n) + f, r);
+          }
+          q += d_q;
+          f += d_f;
+          if (f >= F) {
+            f -= F;
+            ++q;
+          }
         }
       } else {
-        for (int t = tid; t < mres * n; t += kUrThreads) {
-          const int q = t / n, i = t - q * n;
-          if (keep_s[q]) __stcg(R + int64_t(ent_s[q] / L) * n + i, fmaf(-v_s[q], u[i], Es[size_t(q) * es + i]));
+        for (int q = warp; q < mres; q += kUrWarps) {
+          const int p = row_s[q];
+          if (p < 0) continue;
+          const float x = v_s[q];
+          float* const row = R + int64_t(p) * n;
+          for (int i = lane; i < n; i += 32) __stcg(row + i, fmaf(-x, u[i], Es[size_t(q) * es + i]));
         }
       }
       fence_proxy_async_smem();  // generic accesses of Es before the next bulk copies into it
       __syncthreads();
-      if (tid == 0) red_release_add(done_cnt + j, 1u);
+      // nobody else waits for a CTA alone on this atom and the next one
+      if (tid == 0 && (active > 1 || nact > 1)) red_release_add(done_cnt + j, 1u);
       lap(5);
-      if (prefetch) {
-        slot ^= 1;
-        meta_atom = jn;
-      } else {
-        meta_atom = -1;
-      }
+      if (prefetch) slot ^= 1;
+      meta_atom = prefetch ? jn : -1;
     }
   }
   if (timer)
@@ -760,7 +982,15 @@ int update_res_grid_size(int n, int num_sms) {
   return num_sms;  // one CTA per SM: co-resident by construction
 }
 
-size_t update_res_partial_floats(int n, int grid) { return size_t(2) * grid * ur_n4(n); }
+// Zeroed by the launch: the tagged partials (two per CTA, by parity of the power
+// step) and two counters per atom; then the plain partials.
+static size_t ur_zeroed_bytes(int n, int grid, int K) {
+  return (size_t(2) * grid * ur_words(n) + (K + 1) / 2) * sizeof(uint4);
+}
+
+size_t update_res_scratch_bytes(int n, int grid, int K) {
+  return ur_zeroed_bytes(n, grid, K) + size_t(2) * grid * ur_n4(n) * sizeof(float);
+}
 
 cudaError_t launch_residual(const float* Y, int64_t N, int n, const float* D, int K, int L, const int32_t* idx,
                             const float* coef, float* R, int* last, int num_sms, cudaStream_t s) {
@@ -807,41 +1037,14 @@ cudaError_t launch_update_batch(const UpdBatch& batch, GridBarrier* flags, DevSt
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
   if (e != cudaSuccess) return e;
   for (int i = 0; i < batch.ngroups; ++i) {
-    e = cudaMemsetAsync(batch.g[i].sync, 0, size_t(2) * batch.g[i].K * sizeof(unsigned), s);
+    const UpdGroup& g = batch.g[i];
+    // the counters, and the words: no tag of an earlier sweep may be left
+    e = cudaMemsetAsync(g.gw, 0, ur_zeroed_bytes(g.n, g.ctas, g.K), s);
     if (e != cudaSuccess) return e;
   }
   UpdBatch b = batch;
   void* args[] = {(void*)&b, (void*)&flags, (void*)&stats, (void*)&timers};
   return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kUrThreads), args, smem, s);
-}
-
-cudaError_t launch_update_res(float* R, int n, float* D, int K, int L, float* coef, const int* atom_ptr,
-                              const int* entries, int q1_cap, float* gw, unsigned* sync, GridBarrier* flags,
-                              DevStats* stats, int timers, const int* last, int slice_target, int grid,
-                              cudaStream_t s) {
-  const int cap = update_res_capacity(n);
-  if (cap < 16 || grid < 1) return cudaErrorInvalidValue;
-  UpdBatch b;
-  std::memset(&b, 0, sizeof(b));
-  b.ngroups = 1;
-  UpdGroup& g = b.g[0];
-  g.R = R;
-  g.D = D;
-  g.coef = coef;
-  g.atom_ptr = atom_ptr;
-  g.entries = entries;
-  g.last = last;
-  g.gw = gw;
-  g.sync = sync;
-  g.n = n;
-  g.K = K;
-  g.L = L;
-  g.q1_cap = q1_cap;
-  g.cap = cap;
-  g.cta_begin = 0;
-  g.ctas = grid;
-  g.slice_target = slice_target;
-  return launch_update_batch(b, flags, stats, timers, grid, s);
 }
 
 }  // namespace ksvd

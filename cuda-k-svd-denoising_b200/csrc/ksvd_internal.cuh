@@ -128,7 +128,8 @@ cudaError_t launch_accumulate_phases(const DevStats* src, DevStats* dst, cudaStr
 // Dictionary update on a maintained residual (kernels_update_res.cu).
 bool update_res_supported(int n);
 int update_res_grid_size(int n, int num_sms);
-size_t update_res_partial_floats(int n, int grid);
+// Scratch of one problem on `grid` CTAs: partials and counters (the launch zeroes what has to be).
+size_t update_res_scratch_bytes(int n, int grid, int K);
 // last (optional, N ints): the highest atom of each patch's support, -1 if none.
 cudaError_t launch_residual(const float* Y, int64_t N, int n, const float* D, int K, int L, const int32_t* idx,
                             const float* coef, float* R, int* last, int num_sms, cudaStream_t s);
@@ -137,12 +138,11 @@ cudaError_t launch_residual(const float* Y, int64_t N, int n, const float* D, in
 cudaError_t launch_residual_list(const float* Y, int64_t N, int n, const float* D, int K, int L, const int32_t* idx,
                                  const float* coef, float* R, int* last, const int64_t* list,
                                  const unsigned long long* count, int num_sms, cudaStream_t s);
-// sync: 2K unsigned words (zeroed by the launch); gw: update_res_partial_floats.
-// stats receives the counters always, the phase times when timers != 0.
-// One problem of a (multi-problem) update sweep: its buffers (as for
-// launch_update_res; gw: 2 x ctas x round4(n) floats, sync: 2K words, zeroed
-// by the launch), sizes, the resident-column capacity (update_res_capacity(n)
-// or less) and its CTAs [cta_begin, cta_begin + ctas) of the launch.
+// One problem of a (multi-problem) update sweep: its buffers (gw:
+// update_res_scratch_bytes), sizes, the resident-column capacity
+// (update_res_capacity(n) or less), its CTAs [cta_begin, cta_begin + ctas) of
+// the launch and slice_target, the entries per CTA before another CTA joins an
+// atom (<= 0: the default rule).
 struct UpdGroup {
   float* R;
   float* D;
@@ -150,8 +150,7 @@ struct UpdGroup {
   const int* atom_ptr;
   const int* entries;
   const int* last;
-  float* gw;
-  unsigned* sync;
+  void* gw;
   int n, K, L, q1_cap, cap, cta_begin, ctas, slice_target;
 };
 constexpr int kUpdMaxGroups = 64;
@@ -163,15 +162,9 @@ int update_res_capacity(int n);
 // One cooperative launch of `grid` CTAs (one per SM at most) over all groups;
 // each group's CTA range lies in [0, grid); groups whose ranges share CTAs run
 // one after the other on them, in table order.
+// stats receives the counters always, the phase times when timers != 0.
 cudaError_t launch_update_batch(const UpdBatch& batch, GridBarrier* flags, DevStats* stats, int timers, int grid,
                                 cudaStream_t s);
-// last (optional): from launch_residual; a residual row is not stored back by
-// the patch's last atom.  slice_target: entries per CTA before another CTA
-// joins an atom (<= 0: the default, 64).
-cudaError_t launch_update_res(float* R, int n, float* D, int K, int L, float* coef, const int* atom_ptr,
-                              const int* entries, int q1_cap, float* gw, unsigned* sync, GridBarrier* flags,
-                              DevStats* stats, int timers, const int* last, int slice_target, int grid,
-                              cudaStream_t s);
 
 // ---------------------------------------------------------------------------
 // Learned support proposal (kernels_mlp.cu, kernels_omp_restricted.cu).

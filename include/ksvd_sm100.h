@@ -221,9 +221,9 @@ ksvd_status ksvd_profile_reset(ksvd_ctx* ctx);
 int64_t ksvd_launch_count(const ksvd_ctx* ctx);
 /* Wall time (ms) the first CTA of the persistent kernels spent per phase
  * while profiling at level 2 (since the last reset): update [7] slice set-up,
- * [0] wait for the previous atom, [1] column load, [2] local power pass,
- * [3] wait for the other CTAs' partials, [4] partial all-reduce and
- * normalisation, [5] coefficients and residual store; OMP [8] correlation +
+ * [0] wait for the previous atom, [1] column load, [2] local power pass (and
+ * the arrival of the columns), [3] sum of the partials (waiting for the other
+ * CTAs'), [4] normalisation, [5] coefficients and residual store; OMP [8] correlation +
  * argmax, [9] residual update (least squares included for the FP32 kernels),
  * [10] tile load/store, [11] exact re-scores, [12] Cholesky append and solve
  * (tensor-core kernel).  Synchronises the stream. */
