@@ -2,7 +2,7 @@
 //
 // The reference forms all denoised patches D X with one SGEMM, copies them to
 // the host and overlap-adds them in a single host thread.  Here:
-//   col2im_kernel  one CTA per TS x TS pixel tile (TS = 32, 16 or 8; large
+//   col2im_kernel  one CTA per pixel tile (sides of 8 to 64; large
 //                  patches use col2im_direct_kernel, one thread per pixel,
 //                  with the same sums): the denoised patches that
 //                  cover the tile (x_hat_p = sum_s x_s d_s from the compact
@@ -22,28 +22,51 @@
 
 namespace ksvd {
 
-constexpr size_t kCol2imSmemLimit = 100 * 1024;
+// Two CTAs of 1024 threads per SM.  (2048 x 2048 image, 12 x 12 patches at stride 3:
+// 0.57 ms with a 32 x 16 tile, 0.80 with the square 16 x 16 one and 256 threads;
+// 48 x 32 tiles of one CTA per SM take 0.52 there, but lose where a tile of
+// larger patches has few pixels.)
+constexpr size_t kCol2imSmemLimit = 110 * 1024;
+constexpr int kCol2imThreads = 1024;
 
 static int tile_patches_1d(int TS, int ext, int stride) { return (TS + ext - 1) / stride + 1; }
 
-// Tile side of the shared-memory gather: the largest of 32, 16, 8 whose
-// covering patches fit the budget; 0 when none does (large patches), in
+struct Tile {
+  int x, y;
+};
+
+static size_t tile_bytes(const PatchGeom& g, Tile t) {
+  return size_t(tile_patches_1d(t.x, g.ph, g.sh)) * tile_patches_1d(t.y, g.pw, g.sw) * g.n * sizeof(float);
+}
+
+// Pixel tile of the shared-memory gather: of those whose covering patches fit
+// the budget, the one that forms the fewest patches per pixel (each patch is
+// formed once per tile it touches); x = 0 when none fits (large patches), in
 // which case the direct gather runs.
-static int pick_tile(const PatchGeom& g) {
-  const int cands[] = {32, 16, 8};
-  for (int TS : cands) {
-    size_t np = size_t(tile_patches_1d(TS, g.ph, g.sh)) * tile_patches_1d(TS, g.pw, g.sw);
-    if (np * g.n * sizeof(float) <= kCol2imSmemLimit) return TS;
-  }
-  return 0;
+static Tile pick_tile(const PatchGeom& g) {
+  const int sides[] = {64, 48, 32, 24, 16, 8};
+  Tile best{0, 0};
+  double cost = 0.0;
+  for (int tx : sides)
+    for (int ty : sides) {
+      const Tile t{tx, ty};
+      const size_t b = tile_bytes(g, t);
+      if (b > kCol2imSmemLimit) continue;
+      const double c = double(b) / (double(tx) * ty);
+      if (best.x == 0 || c < cost) {
+        best = t;
+        cost = c;
+      }
+    }
+  return best;
 }
 
 constexpr int kDirectThreads = 256;
 
 int col2im_num_tiles(const PatchGeom& g) {
-  const int TS = pick_tile(g);
-  if (TS == 0) return int((int64_t(g.W) * g.H + kDirectThreads - 1) / kDirectThreads);
-  return ((g.W + TS - 1) / TS) * ((g.H + TS - 1) / TS);
+  const Tile t = pick_tile(g);
+  if (t.x == 0) return int((int64_t(g.W) * g.H + kDirectThreads - 1) / kDirectThreads);
+  return ((g.W + t.x - 1) / t.x) * ((g.H + t.y - 1) / t.y);
 }
 
 // ix range covering x: ix*sh <= x < ix*sh + ph, 0 <= ix < nx
@@ -53,15 +76,15 @@ __device__ __forceinline__ int cover_lo(int x, int ext, int stride) {
 }
 __device__ __forceinline__ int cover_hi(int x, int stride, int npos) { return min(npos - 1, x / stride); }
 
-__global__ void __launch_bounds__(256) col2im_kernel(const float* __restrict__ noisy, PatchGeom g, int TS,
+__global__ void __launch_bounds__(kCol2imThreads) col2im_kernel(const float* __restrict__ noisy, PatchGeom g, int TX, int TY,
                                                      const float* __restrict__ D, int K, int L,
                                                      const int32_t* __restrict__ idx, const float* __restrict__ coef,
                                                      float* __restrict__ acc_out, double* __restrict__ partials) {
   extern __shared__ float xs[];
   __shared__ double red[32];
-  const int tx0 = blockIdx.x * TS, ty0 = blockIdx.y * TS;
+  const int tx0 = blockIdx.x * TX, ty0 = blockIdx.y * TY;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  const int tx1 = min(g.W, tx0 + TS) - 1, ty1 = min(g.H, ty0 + TS) - 1;
+  const int tx1 = min(g.W, tx0 + TX) - 1, ty1 = min(g.H, ty0 + TY) - 1;
   const int ixl = cover_lo(tx0, g.ph, g.sh), ixh = cover_hi(tx1, g.sh, g.nx);
   const int iyl = cover_lo(ty0, g.pw, g.sw), iyh = cover_hi(ty1, g.sw, g.ny);
   const int npx = max(0, ixh - ixl + 1), npy = max(0, iyh - iyl + 1);
@@ -118,8 +141,8 @@ __global__ void __launch_bounds__(256) col2im_kernel(const float* __restrict__ n
   }
   __syncthreads();
   double part = 0.0;
-  for (int t = threadIdx.x; t < TS * TS; t += blockDim.x) {
-    const int x = tx0 + t % TS, y = ty0 + t / TS;
+  for (int t = threadIdx.x; t < TX * TY; t += blockDim.x) {
+    const int x = tx0 + t % TX, y = ty0 + t / TX;
     if (x >= g.W || y >= g.H) continue;
     const int ia = max(ixl, cover_lo(x, g.ph, g.sh)), ib = min(ixh, cover_hi(x, g.sh, g.nx));
     const int ja = max(iyl, cover_lo(y, g.pw, g.sw)), jb = min(iyh, cover_hi(y, g.sw, g.ny));
@@ -212,21 +235,20 @@ __global__ void blend_kernel(const float* __restrict__ noisy, PatchGeom g, const
 cudaError_t launch_col2im(const float* noisy, const PatchGeom& g, const float* dict, int K, int L,
                           const int32_t* idx, const float* coef, float* acc, double* partials, int* num_partials,
                           cudaStream_t s) {
-  const int TS = pick_tile(g);
-  if (TS == 0) {
+  const Tile t = pick_tile(g);
+  if (t.x == 0) {
     const int64_t blocks = (int64_t(g.W) * g.H + kDirectThreads - 1) / kDirectThreads;
     col2im_direct_kernel<<<unsigned(blocks), kDirectThreads, 0, s>>>(noisy, g, dict, K, L, idx, coef, acc, partials);
     *num_partials = int(blocks);
     return cudaGetLastError();
   }
-  const size_t np = size_t(tile_patches_1d(TS, g.ph, g.sh)) * tile_patches_1d(TS, g.pw, g.sw);
-  const size_t smem = np * g.n * sizeof(float);
+  const size_t smem = tile_bytes(g, t);
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(col2im_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     if (e != cudaSuccess) return e;
   }
-  dim3 grid((g.W + TS - 1) / TS, (g.H + TS - 1) / TS);
-  col2im_kernel<<<grid, 256, smem, s>>>(noisy, g, TS, dict, K, L, idx, coef, acc, partials);
+  dim3 grid((g.W + t.x - 1) / t.x, (g.H + t.y - 1) / t.y);
+  col2im_kernel<<<grid, kCol2imThreads, smem, s>>>(noisy, g, t.x, t.y, dict, K, L, idx, coef, acc, partials);
   *num_partials = int(grid.x * grid.y);
   return cudaGetLastError();
 }
