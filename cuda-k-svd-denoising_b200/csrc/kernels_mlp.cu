@@ -123,15 +123,19 @@ __global__ void __launch_bounds__(kGThreads) gemm_bf16_kernel(GemmArgs g) {
   const unsigned sbase = smem_u32(gsm);
   auto a_addr = [&](int s) { return sbase + unsigned(s * (a_bytes + b_bytes)); };
   auto b_addr = [&](int s) { return sbase + unsigned(s * (a_bytes + b_bytes) + a_bytes); };
-  const int nk = (g.K + kGKC - 1) / kGKC;
+  // this split's chunks of K
+  const int nk_all = (g.K + kGKC - 1) / kGKC;
+  const int ck0 = int(int64_t(nk_all) * blockIdx.z / gridDim.z);
+  const int nk = int(int64_t(nk_all) * (blockIdx.z + 1) / gridDim.z) - ck0;
+  if (EPI == kEpiF32) g.c_f32 += int64_t(blockIdx.z) * g.split_stride;
   unsigned phase_bits = 0;  // parity of the next completion of each stage's barrier
   unsigned pending = 0;     // stages with a commit not yet waited for (thread 0)
   bool failed = false;
 
   auto load_chunk = [&](int c) {
     const int s = c % kGStages;
-    load_tile<AK>(a_addr(s), g.A, g.lda, m0, g.M, kGM, c * kGKC, g.K, tid);
-    load_tile<BK>(b_addr(s), g.B, g.ldb, n0, g.N, nt, c * kGKC, g.K, tid);
+    load_tile<AK>(a_addr(s), g.A, g.lda, m0, g.M, kGM, (ck0 + c) * kGKC, g.K, tid);
+    load_tile<BK>(b_addr(s), g.B, g.ldb, n0, g.N, nt, (ck0 + c) * kGKC, g.K, tid);
   };
   load_chunk(0);
   cp_async_commit();
@@ -332,7 +336,7 @@ static cudaError_t launch_gemm_t(const GemmArgs& g, cudaStream_t s) {
   auto kern = gemm_bf16_kernel<AK, BK, EPI>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
   if (e != cudaSuccess) return e;
-  dim3 grid((g.M + kGM - 1) / kGM, (g.N + nt - 1) / nt);
+  dim3 grid((g.M + kGM - 1) / kGM, (g.N + nt - 1) / nt, EPI == kEpiF32 && g.splits > 1 ? g.splits : 1);
   kern<<<grid, kGThreads, smem, s>>>(g);
   return cudaGetLastError();
 }
@@ -433,22 +437,35 @@ __global__ void mlp_bce_kernel(const float* __restrict__ Z, int64_t B, int K, in
 }
 
 // Column sums of the first C columns of a B-row BF16 matrix with row stride
-// ld (the bias gradients): FP32 per column.
-__global__ void mlp_colsum_kernel(const __nv_bfloat16* __restrict__ G, int64_t B, int C, int ld,
-                                  float* __restrict__ out) {
+// ld (the bias gradients): FP32 per column and row split (blockIdx.y).
+__global__ void __launch_bounds__(256) mlp_colsum_kernel(const __nv_bfloat16* __restrict__ G, int64_t B, int C, int ld,
+                                                         float* __restrict__ out) {
   __shared__ float part[8][33];
   const int c = blockIdx.x * 32 + (threadIdx.x & 31);
   const int ry = threadIdx.x >> 5;  // 8 row groups
+  const int64_t b0 = B * blockIdx.y / gridDim.y, b1 = B * (blockIdx.y + 1) / gridDim.y;
   float s = 0.0f;
   if (c < C)
-    for (int64_t b = ry; b < B; b += 8) s += __bfloat162float(G[b * ld + c]);
+#pragma unroll 8
+    for (int64_t b = b0 + ry; b < b1; b += 8) s += __bfloat162float(G[b * ld + c]);
   part[ry][threadIdx.x & 31] = s;
   __syncthreads();
   if (ry == 0 && c < C) {
     float t = 0.0f;
     for (int i = 0; i < 8; ++i) t += part[i][threadIdx.x & 31];
-    out[c] = t;
+    out[int64_t(blockIdx.y) * C + c] = t;
   }
+}
+
+// out[i] = sum over the splits of part[split * stride + i], in ascending order.
+__global__ void __launch_bounds__(256) mlp_sum_splits_kernel(const float* __restrict__ part, int splits,
+                                                             int64_t stride, int64_t count, float* __restrict__ out) {
+  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= count) return;
+  float s = 0.0f;
+#pragma unroll 8
+  for (int k = 0; k < splits; ++k) s += part[k * stride + i];
+  out[i] = s;
 }
 
 // Adam (bias-corrected) on the FP32 master parameters.
@@ -503,9 +520,32 @@ cudaError_t launch_mlp_bce(const float* Z, int64_t B, int K, int K16, const int3
   return cudaGetLastError();
 }
 
-cudaError_t launch_mlp_colsum(const __nv_bfloat16* G, int64_t B, int C, int ld, float* out, cudaStream_t s) {
-  mlp_colsum_kernel<<<(C + 31) / 32, 256, 0, s>>>(G, B, C, ld, out);
+cudaError_t launch_mlp_sum_splits(const float* part, int splits, int64_t stride, int64_t count, float* out,
+                                  cudaStream_t s) {
+  mlp_sum_splits_kernel<<<unsigned((count + 255) / 256), 256, 0, s>>>(part, splits, stride, count, out);
   return cudaGetLastError();
+}
+
+// The rows are split so that the columns' few blocks do not leave most SMs
+// idle (512 columns of 4096 rows took 68 us with 16 blocks).
+cudaError_t launch_mlp_colsum(const __nv_bfloat16* G, int64_t B, int C, int ld, float* part, float* out,
+                              cudaStream_t s) {
+  const int splits = int(std::min<int64_t>(kColsumSplits, (B + 31) / 32));
+  mlp_colsum_kernel<<<dim3((C + 31) / 32, splits), 256, 0, s>>>(G, B, C, ld, part);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  return launch_mlp_sum_splits(part, splits, C, C, out, s);
+}
+
+// Splits of K for a gradient GEMM: its tiles are few (4 to 8 for 512 x 512
+// weights) while K is the batch, so K is split over the SMs, at most
+// kMaxGemmSplits ways and at least one chunk each.  (512 x 512, K = 4096 took
+// 653 us unsplit; loss and gradients of 4096 patches: 1.73 ms before, 0.52 with
+// the column sums split as well.)
+int gemm_splits(int M, int N, int K, int num_sms) {
+  const int nt = g_ntile(N), tiles = ((M + kGM - 1) / kGM) * ((N + nt - 1) / nt);
+  const int chunks = (K + kGKC - 1) / kGKC;
+  return std::max(1, std::min(std::min(kMaxGemmSplits, chunks), num_sms / tiles));
 }
 
 cudaError_t launch_mlp_adam(float* w, const float* grad, float* m1, float* m2, int64_t count, float lr, int step,

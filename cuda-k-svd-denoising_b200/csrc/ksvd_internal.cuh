@@ -196,6 +196,8 @@ struct GemmArgs {
   long long ld_aux;
   int32_t* topk;
   int ktop, n_valid;
+  int splits;              // kEpiF32: K in this many parts (0 or 1: one), part i -> c_f32 + i split_stride
+  long long split_stride;
   GridBarrier* flags;
 };
 bool gemm_shape_ok(const GemmArgs& g, bool a_kcontig, bool b_kcontig);
@@ -204,7 +206,14 @@ cudaError_t launch_mlp_input(const float* Y, int64_t B, int n, int np16, const i
                              __nv_bfloat16* X, cudaStream_t s);
 cudaError_t launch_mlp_bce(const float* Z, int64_t B, int K, int K16, const int32_t* sup, int L, const int64_t* rows,
                            __nv_bfloat16* dZ, double* loss_sum, cudaStream_t s);
-cudaError_t launch_mlp_colsum(const __nv_bfloat16* G, int64_t B, int C, int ld, float* out, cudaStream_t s);
+constexpr int kMaxGemmSplits = 16, kColsumSplits = 16;
+int gemm_splits(int M, int N, int K, int num_sms);
+// out[i] = sum_k part[k stride + i], i < count.
+cudaError_t launch_mlp_sum_splits(const float* part, int splits, int64_t stride, int64_t count, float* out,
+                                  cudaStream_t s);
+// part: kColsumSplits x C scratch.
+cudaError_t launch_mlp_colsum(const __nv_bfloat16* G, int64_t B, int C, int ld, float* part, float* out,
+                              cudaStream_t s);
 cudaError_t launch_mlp_adam(float* w, const float* grad, float* m1, float* m2, int64_t count, float lr, int step,
                             cudaStream_t s);
 cudaError_t launch_mlp_to_bf16(const float* w, int rows, int cols, int rows_pad, int ld, __nv_bfloat16* out,

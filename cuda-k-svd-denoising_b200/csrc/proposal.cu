@@ -97,7 +97,7 @@ ksvd_status reset_optimizer(ksvd_ctx* c, const Bufs& b) {
 // Activations of one batch of B rows.
 struct Acts {
   __nv_bfloat16 *X, *H1, *H2, *dZ3, *dZ2, *dZ1;
-  float *Z1, *Z2, *Z3, *tmp;
+  float *Z1, *Z2, *Z3, *tmp, *part;
 };
 
 ksvd_status acts_of(ksvd_ctx* c, int64_t B, bool train, Acts* a) {
@@ -114,6 +114,8 @@ ksvd_status acts_of(ksvd_ctx* c, int64_t B, bool train, Acts* a) {
     KSVD_TRY(wsT(c, "prop_tdZ2", size_t(B) * kH, &a->dZ2));
     KSVD_TRY(wsT(c, "prop_tdZ1", size_t(B) * kH, &a->dZ1));
     KSVD_TRY(wsT(c, "prop_tmp", size_t(std::max(kH * P.n16, P.K16 * kH)), &a->tmp));
+    // split gradients: one weight matrix (or bias) at a time
+    KSVD_TRY(wsT(c, "prop_part", size_t(ksvd::kMaxGemmSplits) * kH * std::max(kH, P.n16), &a->part));
   }
   return KSVD_OK;
 }
@@ -173,6 +175,24 @@ ksvd_status forward(ksvd_ctx* c, const Bufs& b, const Acts& a, int64_t B, bool t
   return KSVD_OK;
 }
 
+// A weight gradient: the GEMM of g, K split where that fills the SMs, its parts
+// summed into g.c_f32 (dense rows of g.ldc_f32).
+ksvd_status grad_gemm(ksvd_ctx* c, ksvd::GemmArgs g, float* part, const char* what) {
+  float* const out = g.c_f32;
+  const int64_t count = int64_t(g.M) * g.ldc_f32;
+  g.splits = ksvd::gemm_splits(g.M, g.N, g.K, c->num_sms);
+  if (g.splits > 1) {
+    g.c_f32 = part;
+    g.split_stride = count;
+  }
+  KSVD_CU(c, ksvd::launch_gemm(g, false, false, ksvd::kEpiF32, c->stream), what);
+  if (g.splits > 1) {
+    KSVD_CU(c, ksvd::launch_mlp_sum_splits(part, g.splits, count, count, out, c->stream), what);
+    c->launch_count += 1;
+  }
+  return KSVD_OK;
+}
+
 // Loss gradient and backward pass into b.g (parameter order of Offs).
 // sup/rows: the supports of the batch rows (see launch_mlp_bce).
 ksvd_status backward(ksvd_ctx* c, const Bufs& b, const Acts& a, int64_t B, const int32_t* sup,
@@ -192,11 +212,11 @@ ksvd_status backward(ksvd_ctx* c, const Bufs& b, const Acts& a, int64_t B, const
   g.K = int(B);
   g.c_f32 = (P.K == P.K16) ? b.g + o.W3 : a.tmp;
   g.ldc_f32 = kH;
-  KSVD_CU(c, ksvd::launch_gemm(g, false, false, ksvd::kEpiF32, c->stream), "proposal dW3");
+  KSVD_TRY(grad_gemm(c, g, a.part, "proposal dW3"));
   if (P.K != P.K16)
     KSVD_CU(c, cudaMemcpyAsync(b.g + o.W3, a.tmp, size_t(P.K) * kH * 4, cudaMemcpyDeviceToDevice, c->stream),
             "proposal dW3");
-  KSVD_CU(c, ksvd::launch_mlp_colsum(a.dZ3, B, P.K, P.K16, b.g + o.b3, c->stream), "proposal db3");
+  KSVD_CU(c, ksvd::launch_mlp_colsum(a.dZ3, B, P.K, P.K16, a.part, b.g + o.b3, c->stream), "proposal db3");
   // dZ2 = (dZ3 W3) * GELU'(Z2)
   g = gemm0(c);
   g.A = a.dZ3;
@@ -222,8 +242,8 @@ ksvd_status backward(ksvd_ctx* c, const Bufs& b, const Acts& a, int64_t B, const
   g.K = int(B);
   g.c_f32 = b.g + o.W2;
   g.ldc_f32 = kH;
-  KSVD_CU(c, ksvd::launch_gemm(g, false, false, ksvd::kEpiF32, c->stream), "proposal dW2");
-  KSVD_CU(c, ksvd::launch_mlp_colsum(a.dZ2, B, kH, kH, b.g + o.b2, c->stream), "proposal db2");
+  KSVD_TRY(grad_gemm(c, g, a.part, "proposal dW2"));
+  KSVD_CU(c, ksvd::launch_mlp_colsum(a.dZ2, B, kH, kH, a.part, b.g + o.b2, c->stream), "proposal db2");
   // dZ1 = (dZ2 W2) * GELU'(Z1)
   g = gemm0(c);
   g.A = a.dZ2;
@@ -249,10 +269,10 @@ ksvd_status backward(ksvd_ctx* c, const Bufs& b, const Acts& a, int64_t B, const
   g.K = int(B);
   g.c_f32 = (P.n == P.n16) ? b.g + o.W1 : a.tmp;
   g.ldc_f32 = P.n16;
-  KSVD_CU(c, ksvd::launch_gemm(g, false, false, ksvd::kEpiF32, c->stream), "proposal dW1");
+  KSVD_TRY(grad_gemm(c, g, a.part, "proposal dW1"));
   if (P.n != P.n16) KSVD_CU(c, ksvd::launch_mlp_unpad(a.tmp, kH, P.n, P.n16, b.g + o.W1, c->stream), "proposal dW1");
-  KSVD_CU(c, ksvd::launch_mlp_colsum(a.dZ1, B, kH, kH, b.g + o.b1, c->stream), "proposal db1");
-  c->launch_count += 11;
+  KSVD_CU(c, ksvd::launch_mlp_colsum(a.dZ1, B, kH, kH, a.part, b.g + o.b1, c->stream), "proposal db1");
+  c->launch_count += 14;
   return KSVD_OK;
 }
 
