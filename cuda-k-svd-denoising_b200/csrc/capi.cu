@@ -301,10 +301,11 @@ ksvd_status omp_form(ksvd_ctx* c, const float* d_patches, int64_t N, const float
   if (precision == KSVD_PREC_BF16_LEARNED) return omp_learned_impl(c, d_patches, N, d_dict, gram, d_idx, d_coef);
   Prof pr(c, "omp", 1);
   ksvd::DevStats* ph = c->profiling >= 2 ? c->d_phase : nullptr;
-  // The tensor-core forms need the 16-bit dictionary in shared memory (atoms
-  // <= 256); beyond that, and for the FP32 form, the FP32 kernels run: the
+  // Every form runs on the tensor cores, with the 16-bit dictionary in shared
+  // memory where it fits (up to 256 atoms), else streamed (up to 512 atoms);
+  // beyond that (and beyond 16 atoms per patch) the FP32 kernels run: the
   // resident-dictionary one when it fits, else the streamed one.
-  // Before an update sweep the 16-bit kernels also write the sweep's residual
+  // Before an update sweep the tensor-core kernels also write the sweep's residual
   // rows (the same buffers and arithmetic as launch_residual); patches that
   // took fewer than L atoms are listed and formed after them.
   float* resid = nullptr;
@@ -327,21 +328,24 @@ ksvd_status omp_form(ksvd_ctx* c, const float* d_patches, int64_t N, const float
     c->resid_fused = true;
     return KSVD_OK;
   };
-  if (precision != KSVD_PREC_FP32 && ksvd::omp_tc_supported(n, K, L)) {
+  const ksvd::TcForm form = precision == KSVD_PREC_FP32           ? ksvd::TcForm::kFp32
+                            : precision == KSVD_PREC_FP16_RESCORE ? ksvd::TcForm::kFp16
+                                                                  : ksvd::TcForm::kBf16;
+  if (ksvd::omp_tc_supported(n, K, L)) {
     if (for_update) KSVD_TRY(fused_buffers());
     KSVD_CU(c,
             ksvd::launch_omp_tc(d_patches, N, n, d_dict, gram, K, L, d_idx, d_coef, c->num_sms,
-                                precision == KSVD_PREC_FP16_RESCORE ? 1 : 0, c->d_flags, ph, c->stream, resid, last,
+                                form, c->d_flags, ph, c->stream, resid, last,
                                 fix, nfix),
             "omp (tensor cores)");
     if (for_update) KSVD_TRY(listed_rows());
-  } else if (precision != KSVD_PREC_FP32 && ksvd::omp_tcb_supported(n, K, L)) {
+  } else if (ksvd::omp_tcb_supported(n, K, L)) {
     void* scratch = nullptr;
-    KSVD_TRY(ws(c, "tcb_scratch", ksvd::omp_tcb_scratch_bytes(n, K), &scratch));
+    KSVD_TRY(ws(c, "tcb_scratch", ksvd::omp_tcb_scratch_bytes(n, K, form, c->num_sms), &scratch));
     if (for_update) KSVD_TRY(fused_buffers());
     KSVD_CU(c,
             ksvd::launch_omp_tcb(d_patches, N, n, d_dict, gram, K, L, d_idx, d_coef, c->num_sms,
-                                 precision == KSVD_PREC_FP16_RESCORE ? 1 : 0, scratch, c->d_flags, ph, c->stream,
+                                 form, scratch, c->d_flags, ph, c->stream,
                                  resid, last, fix, nfix),
             "omp (tensor cores, streamed dictionary)");
     if (for_update) KSVD_TRY(listed_rows());

@@ -19,6 +19,16 @@
 //     pseudo-inverse, :269-339), forms the FP32 residual y - D_S g and its
 //     norm (:352-393; stop when below 1e-3, :218) and writes the residual as
 //     BF16 into the A operand of the next step.
+//
+// The plain FP32 form (F32) takes the argmax of the FP32 correlations that
+// kernels_omp.cu forms, sum_k fma(d_a[k], r[k]) with k ascending.  Its FP16
+// correlation only narrows the atoms down: those that could hold the largest
+// FP32 value within both rounding errors are scored with that very sum, so the
+// codes are the ones of kernels_omp.cu.  The tile keeps the FP32 residual in
+// shared memory in the place of the patches, which are read again from L2.
+// (2048 x 2048 image, 12 x 12 patches, 256 atoms, L = 5: 4.3 ms, 7.7 with the
+// SIMT correlation, which is bound by the FP32 pipe; 1.4 atoms scored per patch
+// and step.  Bound now by the latency of the epilogue, like the 16-bit forms.)
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -140,7 +150,11 @@ __host__ __device__ inline TcLayout tc_layout(int n, int K, int L) {
   return o;
 }
 
-template <bool F16>
+// F32: rounding of the FP32 sums (the scored one, the atom sums, the mean part)
+// per feature, in units of |r| |d|.
+constexpr float kF32Slack = 4.0f / 16777216.0f;
+
+template <bool F16, bool F32>
 __global__ void __launch_bounds__(kTcThreads, 1)
     omp_tc_kernel(const float* __restrict__ Y, int64_t N, int n, const float* __restrict__ D,
                   const double* __restrict__ Gram, int K, int L, int32_t* __restrict__ idx_out,
@@ -184,21 +198,53 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     mbar_init(mbar, 1);
     fence_mbar_init();
   }
-  for (int t = tid; t < Kp * nkc; t += kTcThreads) {
-    const int a = t / nkc, kc = t - a * nkc;
-    unsigned short h[8];
+  // the 16-bit dictionary D * dinv
+  auto convert = [&](float dinv) {
+    for (int t = tid; t < Kp * nkc; t += kTcThreads) {
+      const int a = t / nkc, kc = t - a * nkc;
+      unsigned short h[8];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const int k = kc * 8 + e;
-      h[e] = Op16<F16>::cvt((a < K && k < n) ? __ldg(D + int64_t(a) * n + k) : 0.0f);
+      for (int e = 0; e < 8; ++e) {
+        const int k = kc * 8 + e;
+        const float d = (a < K && k < n) ? __ldg(D + int64_t(a) * n + k) : 0.0f;
+        h[e] = Op16<F16>::cvt(F32 ? d * dinv : d);
+      }
+      store8(Bt + canon_off(a, kc * 8, Kp), h);
     }
-    store8(Bt + canon_off(a, kc * 8, Kp), h);
+  };
+  if constexpr (!F32) convert(1.0f);
+  __shared__ unsigned s_dmax;  // F32: bits of the largest |d_a|^2 (a NaN's are larger than any number's)
+  if constexpr (F32) {
+    if (tid == 0) s_dmax = 0u;
+    __syncthreads();
   }
   for (int a = tid; a < Kp; a += kTcThreads) {
-    float sa = 0.0f;
+    float sa = 0.0f, sq = 0.0f;
     if (a < K)
-      for (int k = 0; k < n; ++k) sa += __ldg(D + int64_t(a) * n + k);
+      for (int k = 0; k < n; ++k) {
+        const float d = __ldg(D + int64_t(a) * n + k);
+        sa += d;
+        if constexpr (F32) sq = fmaf(d, d, sq);
+      }
     asum[a] = sa;
+    if constexpr (F32) atomicMax(&s_dmax, __float_as_uint(sq) & 0x7fffffffu);
+  }
+  // F32 takes dictionaries of any scale: the 16-bit one is D / dscale (a power
+  // of two, atoms of norm below 1); out of the range where that is exact
+  // enough, dmax is infinite and every atom is scored
+  float dmax = 1.0f, dscale = 1.0f;
+  if constexpr (F32) {
+    __syncthreads();
+    dmax = sqrtf(__uint_as_float(s_dmax));
+    if (dmax > 1e-15f && dmax < 1e15f) {
+      int e;
+      frexpf(dmax, &e);
+      dscale = ldexpf(1.0f, e);
+      dmax *= 1.0001f;
+    } else {
+      dmax = __int_as_float(0x7f800000);
+    }
+    convert(1.0f / dscale);
   }
   fence_proxy_async_smem();
   tc_fence_before();
@@ -236,6 +282,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       tmark = t;
     }
   };
+  const float slack = kF32Slack * float(n);
+  const bool y_vec4 = (n & 3) == 0 && (reinterpret_cast<uintptr_t>(Y) & 15) == 0;
   int nscored = 0;
   int64_t p0 = 0;  // first patch of the current tile
   // chunk kc of patch m's residual row into R_out
@@ -303,6 +351,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         P.rmean = mean;
         P.rscale = pow2_scale(fmaxf(fmaxf(X.part[0].x, X.part[1].x), fmaxf(X.part[2].x, X.part[3].x)));
         P.rnorm = sqrtf((X.part[0].y + X.part[1].y) + (X.part[2].y + X.part[3].y));
+        if constexpr (F32) P.rnorm = dmax * (Op16<F16>::err * P.rnorm + slack * sqrtf(float(yy)));
       }
     }
     __syncthreads();
@@ -346,7 +395,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       lap(8);
       // ---- this quarter's correlations (tensor part + exact mean part) -----
       const bool done = P.done != 0;
-      const float rmean = P.rmean, rscale = P.rscale;
+      const float rmean = P.rmean, rscale = F32 ? P.rscale * dscale : P.rscale;
       float cv[64];  // up to 64 columns per quarter (Kp <= 256)
       float qmax = -1.0f;
       if (c_lo < Kp) {
@@ -377,11 +426,12 @@ __global__ void __launch_bounds__(kTcThreads, 1)
           float gmax = X.qmax[0];
 #pragma unroll
           for (int j = 1; j < kTcQ; ++j) gmax = fmaxf(gmax, X.qmax[j]);
-          const float thr = gmax - 2.0f * Op16<F16>::err * P.rnorm;
+          // (F32: rnorm is the whole error bound; where it is no number, all atoms)
+          const float thr = gmax - 2.0f * (F32 ? P.rnorm : Op16<F16>::err * P.rnorm);
 #pragma unroll
           for (int i = 0; i < 64; ++i) {
             const int a = c_lo + i;
-            if (a < c_hi && a < K && cv[i] >= thr) mask |= 1ull << i;
+            if (a < c_hi && a < K && (F32 ? !(cv[i] < thr) : cv[i] >= thr)) mask |= 1ull << i;
           }
         }
         X.qmask[q] = mask;
@@ -433,7 +483,39 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             }
           }
           __syncthreads();
-          for (int t = grp; t < rh - rb; t += kTcThreads / 4) {
+          if constexpr (F32) {  // a thread per candidate: the sum of kernels_omp.cu
+            for (int t = tid; t < rh - rb; t += kTcThreads) {
+              const int v = lpk[t];
+              const int ps = v >> 24, a = v & 0xFFFFFF;
+              const float* rr = Ys + ps * ysn;
+              float c = 0.0f;
+              if (d_vec4) {
+                const float4* dr = reinterpret_cast<const float4*>(D + int64_t(a) * n);
+                const int n4 = n / 4;
+                constexpr int kU = 9;  // loads in flight
+                for (int k0 = 0; k0 < n4; k0 += kU) {
+                  float4 dv[kU];
+#pragma unroll
+                  for (int u = 0; u < kU; ++u) dv[u] = __ldg(dr + min(k0 + u, n4 - 1));
+#pragma unroll
+                  for (int u = 0; u < kU; ++u)
+                    if (k0 + u < n4) {
+                      const float* rv = rr + 4 * (k0 + u);
+                      c = fmaf(dv[u].x, rv[0], c);
+                      c = fmaf(dv[u].y, rv[1], c);
+                      c = fmaf(dv[u].z, rv[2], c);
+                      c = fmaf(dv[u].w, rv[3], c);
+                    }
+                }
+              } else {
+#pragma unroll 8
+                for (int k = 0; k < n; ++k) c = fmaf(__ldg(D + int64_t(a) * n + k), rr[k], c);
+              }
+              lcs[t] = double(fabsf(c));
+              ++nscored;
+            }
+          }
+          for (int t = grp; !F32 && t < rh - rb; t += kTcThreads / 4) {
             const int v = lpk[t];
             const int ps = v >> 24, a = v & 0xFFFFFF;
             const float* yrs = Ys + ps * ysn;
@@ -487,11 +569,43 @@ __global__ void __launch_bounds__(kTcThreads, 1)
               if (aca > X.best || (aca == X.best && a < X.best_a)) {
                 X.best = aca;
                 X.best_a = a;
-                X.best_b = lbs[t - rb];
+                if constexpr (!F32) X.best_b = lbs[t - rb];
               }
             }
           }
           __syncthreads();
+        }
+      }
+      if constexpr (F32) {
+        // b = d_a . y of the selected atoms (FP64), a warp per patch, four at a time
+        __syncthreads();
+        constexpr int kPW = 4;
+        for (int i0 = 0; i0 < kTcTile / (kTcThreads / 32); i0 += kPW) {
+          double bp[kPW];
+          int av[kPW];
+#pragma unroll
+          for (int i = 0; i < kPW; ++i) {
+            const int pm = warp * (kTcTile / (kTcThreads / 32)) + i0 + i;
+            const int ba = xq[pm].best_a;
+            av[i] = pp[pm].done ? -1 : ((ba >= 0 && ba < K) ? ba : 0);
+            bp[i] = 0.0;
+          }
+          for (int k = lane; k < n; k += 32) {
+            float dv[kPW], yv[kPW];
+#pragma unroll
+            for (int i = 0; i < kPW; ++i) {
+              const int pm = warp * (kTcTile / (kTcThreads / 32)) + i0 + i;
+              dv[i] = av[i] >= 0 ? __ldg(D + int64_t(av[i]) * n + k) : 0.0f;
+              yv[i] = av[i] >= 0 ? __ldg(Y + (p0 + pm) * n + k) : 0.0f;
+            }
+#pragma unroll
+            for (int i = 0; i < kPW; ++i) bp[i] = fma(double(dv[i]), double(yv[i]), bp[i]);
+          }
+#pragma unroll
+          for (int i = 0; i < kPW; ++i) {
+            const double t = warp_sum(bp[i]);
+            if (lane == 0) xq[warp * (kTcTile / (kTcThreads / 32)) + i0 + i].best_b = t;
+          }
         }
       }
       __syncthreads();
@@ -564,7 +678,19 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
             const int kk = kc * 8 + e;
-            r[e] = (kk < n) ? yr[kk] : 0.0f;
+            r[e] = (!F32 && kk < n) ? yr[kk] : 0.0f;
+          }
+          if constexpr (F32) {  // the patch again, from L2
+            const float* yg = Y + (p0 + m) * n + kc * 8;
+            if (y_vec4 && kc * 8 + 8 <= n) {
+              const float4 y0 = __ldg(reinterpret_cast<const float4*>(yg));
+              const float4 y1 = __ldg(reinterpret_cast<const float4*>(yg) + 1);
+              r[0] = y0.x, r[1] = y0.y, r[2] = y0.z, r[3] = y0.w;
+              r[4] = y1.x, r[5] = y1.y, r[6] = y1.z, r[7] = y1.w;
+            } else {
+#pragma unroll
+              for (int e = 0; e < 8; ++e) r[e] = (kc * 8 + e < n) ? __ldg(yg + e) : 0.0f;
+            }
           }
           if (d_vec4 && kc * 8 + 8 <= n) {
             // the chunk of every support atom is loaded before it is used
@@ -606,6 +732,10 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             }
           }
           if (fin) store_row_chunk(kc, r);
+          if constexpr (F32)
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+              if (kc * 8 + e < n) Ys[m * ysn + kc * 8 + e] = r[e];
           unsigned short h[8];
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
@@ -628,6 +758,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
           tc += part[j].y;
         }
         P.rnorm = sqrtf(tc);
+        if constexpr (F32) P.rnorm = dmax * (Op16<F16>::err * P.rnorm + slack * sqrtf(tn));
         if (sqrtf(tn) < 1e-3f) P.done = 1;
       }
       lap(9);
@@ -666,24 +797,19 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 
 size_t omp_tc_smem_bytes(int n, int K, int L) { return tc_layout(n, K, L).total; }
 
-template __global__ void omp_tc_kernel<false>(const float*, int64_t, int, const float*, const double*, int, int,
-                                              int32_t*, float*, int64_t, int, float*, int*, int64_t*,
-                                              unsigned long long*, int, GridBarrier*, DevStats*);
-template __global__ void omp_tc_kernel<true>(const float*, int64_t, int, const float*, const double*, int, int,
-                                             int32_t*, float*, int64_t, int, float*, int*, int64_t*,
-                                             unsigned long long*, int, GridBarrier*, DevStats*);
-
 bool omp_tc_supported(int n, int K, int L) {
   return L >= 1 && L <= kTcLMax && n >= 1 && K >= 1 && tc_al(K, 16) <= 256 &&
          omp_tc_smem_bytes(n, K, L) <= 232448 - 256;
 }
 
 cudaError_t launch_omp_tc(const float* patches, int64_t N, int n, const float* dict, const double* gram, int K, int L,
-                          int32_t* idx, float* coef, int num_sms, int fp16, GridBarrier* flags, DevStats* stats,
+                          int32_t* idx, float* coef, int num_sms, TcForm form, GridBarrier* flags, DevStats* stats,
                           cudaStream_t s, float* resid_out, int* last_out, int64_t* fix_list,
                           unsigned long long* fix_count) {
   const size_t smem = omp_tc_smem_bytes(n, K, L);
-  auto kern = fp16 ? omp_tc_kernel<true> : omp_tc_kernel<false>;
+  auto kern = form == TcForm::kFp32  ? omp_tc_kernel<true, true>
+              : form == TcForm::kFp16 ? omp_tc_kernel<true, false>
+                                      : omp_tc_kernel<false, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
   if (e != cudaSuccess) return e;
   const int64_t ntiles = (N + kTcTile - 1) / kTcTile;

@@ -19,6 +19,13 @@
 //     holding it in registers;
 //   * the FP32 patches stay in global memory (L2) instead of shared memory:
 //     the exact re-scores and the residual read them there.
+//
+// The plain FP32 form (F32) is the one of kernels_omp_tc.cu: the FP16
+// correlation narrows the atoms down to those that could hold the largest FP32
+// correlation, which are scored with the FP32 sum of kernels_omp_stream.cu, so
+// the codes are that kernel's.  The tile's FP32 residual rows are kept in a
+// scratch buffer (they stay in L2).  (1024 x 1024 image, 16 x 16 patches, 512
+// atoms, L = 8: 10.0 ms, 29.4 with the SIMT correlation.)
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -56,6 +63,8 @@ struct TbOp<true> {
   static constexpr unsigned fmt = 0u;
   static constexpr float err = kTbErrF16;
 };
+
+constexpr float kTbF32Slack = 4.0f / 16777216.0f;  // kF32Slack of kernels_omp_tc.cu
 
 __device__ __forceinline__ void tb_store8(unsigned char* dst, const unsigned short (&h)[8]) {
   uint4 v;
@@ -134,11 +143,48 @@ __host__ __device__ inline TbLayout tb_layout(int n, int K, int L) {
   return o;
 }
 
+// F32 takes dictionaries of any scale: the 16-bit one is D / scale (a power of
+// two, atoms of norm below 1); outside the range where that is exact enough,
+// `dmax` is infinite and every atom is scored.
+struct TbScale {
+  float dmax, scale;
+};
+
+__device__ __forceinline__ TbScale tb_scale(unsigned sq_bits) {
+  TbScale t;
+  t.dmax = sqrtf(__uint_as_float(sq_bits));
+  t.scale = 1.0f;
+  if (t.dmax > 1e-15f && t.dmax < 1e15f) {
+    int e;
+    frexpf(t.dmax, &e);
+    t.scale = ldexpf(1.0f, e);
+    t.dmax *= 1.0001f;
+  } else {
+    t.dmax = __int_as_float(0x7f800000);
+  }
+  return t;
+}
+
+// Bits of the largest |d_a|^2 (a NaN's are larger than any number's); a warp per atom.
+__global__ void tb_norm_kernel(const float* __restrict__ D, int K, int n, unsigned* __restrict__ sq_max) {
+  const int a = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (a >= K) return;
+  float sq = 0.0f;
+  for (int k = lane; k < n; k += 32) {
+    const float d = __ldg(D + int64_t(a) * n + k);
+    sq = fmaf(d, d, sq);
+  }
+  sq = warp_sum(sq);
+  if (lane == 0) atomicMax(sq_max, __float_as_uint(sq) & 0x7fffffffu);
+}
+
 // The 16-bit dictionary (Kp x np16, canonical K-major layout, zero padding)
 // and the atom sums in global memory.
 template <bool F16>
 __global__ void tb_prep_kernel(const float* __restrict__ D, int K, int n, int Kp, int np16,
-                               unsigned char* __restrict__ Bg, float* __restrict__ asum) {
+                               unsigned char* __restrict__ Bg, float* __restrict__ asum,
+                               const unsigned* __restrict__ sq_max) {
+  const float dinv = sq_max ? 1.0f / tb_scale(*sq_max).scale : 1.0f;
   const int nkc = np16 / 8;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < Kp * nkc; t += gridDim.x * blockDim.x) {
     const int a = t / nkc, kc = t - a * nkc;
@@ -146,7 +192,7 @@ __global__ void tb_prep_kernel(const float* __restrict__ D, int K, int n, int Kp
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       const int k = kc * 8 + e;
-      h[e] = TbOp<F16>::cvt((a < K && k < n) ? __ldg(D + int64_t(a) * n + k) : 0.0f);
+      h[e] = TbOp<F16>::cvt((a < K && k < n) ? __ldg(D + int64_t(a) * n + k) * dinv : 0.0f);
     }
     tb_store8(Bg + canon_off(a, kc * 8, Kp), h);
   }
@@ -158,14 +204,15 @@ __global__ void tb_prep_kernel(const float* __restrict__ D, int K, int n, int Kp
   }
 }
 
-template <bool F16>
+template <bool F16, bool F32>
 __global__ void __launch_bounds__(kTbThreads, 1)
     omp_tcb_kernel(const float* __restrict__ Y, int64_t N, int n, const float* __restrict__ D,
                    const unsigned char* __restrict__ Bg, const float* __restrict__ asum_g,
                    const double* __restrict__ Gram, int K, int L, int32_t* __restrict__ idx_out,
                    float* __restrict__ coef_out, int64_t ntiles, int d_vec4, float* __restrict__ R_out,
                    int* __restrict__ last_out, int64_t* __restrict__ fix_list,
-                   unsigned long long* __restrict__ fix_count, int r_vec4, GridBarrier* flags, DevStats* stats) {
+                   unsigned long long* __restrict__ fix_count, int r_vec4, const unsigned* __restrict__ sq_max,
+                   float* __restrict__ Rg, GridBarrier* flags, DevStats* stats) {
   extern __shared__ __align__(128) unsigned char smem[];
   const TbLayout lo = tb_layout(n, K, L);
   unsigned char* ring = smem + lo.off_ring;
@@ -227,6 +274,14 @@ __global__ void __launch_bounds__(kTbThreads, 1)
   double* Lp = Lc + m * tri;
   auto Lat = [&](int i, int j) -> double& { return Lp[i * (i + 1) / 2 + j]; };
   int nscored = 0;
+  float dmax = 1.0f, dscale = 1.0f;
+  if constexpr (F32) {
+    const TbScale t = tb_scale(*sq_max);
+    dmax = t.dmax;
+    dscale = t.scale;
+  }
+  const float slack = kTbF32Slack * float(n);
+  float* const Rt = F32 ? Rg + size_t(blockIdx.x) * kTbTile * n : nullptr;  // this tile's residual rows
 
   // thread 0: one step of MMAs over all K-slices, streaming the slices
   auto mma_step = [&]() -> bool {
@@ -315,6 +370,7 @@ __global__ void __launch_bounds__(kTbThreads, 1)
         P.rmean = mean;
         P.rscale = tb_pow2_scale(fmaxf(fmaxf(X.part[0].x, X.part[1].x), fmaxf(X.part[2].x, X.part[3].x)));
         P.rnorm = sqrtf((X.part[0].y + X.part[1].y) + (X.part[2].y + X.part[3].y));
+        if constexpr (F32) P.rnorm = dmax * (TbOp<F16>::err * P.rnorm + slack * sqrtf(float(yy)));
       }
     }
     __syncthreads();
@@ -348,7 +404,7 @@ __global__ void __launch_bounds__(kTbThreads, 1)
       tc_fence_after();
       // ---- pass 1: this quarter's largest |c| -------------------------------
       const bool done = P.done != 0;
-      const float rmean = P.rmean, rscale = P.rscale;
+      const float rmean = P.rmean, rscale = F32 ? P.rscale * dscale : P.rscale;
       float qmax = -1.0f;
       for (int c0 = c_lo; c0 < c_hi; c0 += 16) {
         float v[16];
@@ -368,7 +424,8 @@ __global__ void __launch_bounds__(kTbThreads, 1)
         float gmax = X.qmax[0];
 #pragma unroll
         for (int j = 1; j < kTbQ; ++j) gmax = fmaxf(gmax, X.qmax[j]);
-        const float thr = gmax - 2.0f * TbOp<F16>::err * P.rnorm;
+        // (F32: rnorm is the whole error bound; where it is no number, all atoms)
+        const float thr = gmax - 2.0f * (F32 ? P.rnorm : TbOp<F16>::err * P.rnorm);
         for (int c0 = c_lo; c0 < c_hi; c0 += 16) {
           float v[16];
           tc_ld16(lane_addr + unsigned(c0), v);
@@ -378,7 +435,8 @@ __global__ void __launch_bounds__(kTbThreads, 1)
             for (int i = 0; i < 16; ++i) {
               const int a = c0 + i;
               const int bit = a - c_lo;
-              if (a < K && fabsf(fmaf(rmean, asum[a], v[i] * rscale)) >= thr) {
+              const float c = fabsf(fmaf(rmean, asum[a], v[i] * rscale));
+              if (a < K && (F32 ? !(c < thr) : c >= thr)) {
                 if (bit < 64)
                   mk0 |= 1ull << bit;
                 else
@@ -433,7 +491,42 @@ __global__ void __launch_bounds__(kTbThreads, 1)
               }
           }
           __syncthreads();
-          for (int t = grp; t < rh - rb; t += kTbThreads / 4) {
+          if constexpr (F32) {  // a thread per candidate: the sum of kernels_omp_stream.cu
+            for (int t = tid; t < rh - rb; t += kTbThreads) {
+              const int v = lpk[t];
+              const int ps = v >> 24, a = v & 0xFFFFFF;
+              const float* rr = step == 0 ? Y + (p0 + ps) * n : Rt + size_t(ps) * n;
+              float c = 0.0f;
+              if (d_vec4) {
+                const float4* dr = reinterpret_cast<const float4*>(D + int64_t(a) * n);
+                const float4* r4 = reinterpret_cast<const float4*>(rr);
+                const int n4 = n / 4;
+                constexpr int kU = 8;  // loads in flight of either row
+                for (int k0 = 0; k0 < n4; k0 += kU) {
+                  float4 dv[kU], rv[kU];
+#pragma unroll
+                  for (int u = 0; u < kU; ++u) {
+                    dv[u] = __ldg(dr + min(k0 + u, n4 - 1));
+                    rv[u] = __ldcg(r4 + min(k0 + u, n4 - 1));
+                  }
+#pragma unroll
+                  for (int u = 0; u < kU; ++u)
+                    if (k0 + u < n4) {
+                      c = fmaf(dv[u].x, rv[u].x, c);
+                      c = fmaf(dv[u].y, rv[u].y, c);
+                      c = fmaf(dv[u].z, rv[u].z, c);
+                      c = fmaf(dv[u].w, rv[u].w, c);
+                    }
+                }
+              } else {
+#pragma unroll 8
+                for (int k = 0; k < n; ++k) c = fmaf(__ldg(D + int64_t(a) * n + k), __ldcg(rr + k), c);
+              }
+              lcs[t] = double(fabsf(c));
+              ++nscored;
+            }
+          }
+          for (int t = grp; !F32 && t < rh - rb; t += kTbThreads / 4) {
             const int v = lpk[t];
             const int ps = v >> 24, a = v & 0xFFFFFF;
             const float* yrs = Y + (p0 + ps) * n;
@@ -476,11 +569,42 @@ __global__ void __launch_bounds__(kTbThreads, 1)
               if (aca > X.best || (aca == X.best && a < X.best_a)) {
                 X.best = aca;
                 X.best_a = a;
-                X.best_b = lbs[t - rb];
+                if constexpr (!F32) X.best_b = lbs[t - rb];
               }
             }
           }
           __syncthreads();
+        }
+      }
+      if constexpr (F32) {
+        // b = d_a . y of the selected atoms (FP64), a warp per patch, four at a time
+        __syncthreads();
+        constexpr int kPW = 4, kPer = kTbTile / (kTbThreads / 32);
+        for (int i0 = 0; i0 < kPer; i0 += kPW) {
+          double bp[kPW];
+          int av[kPW];
+#pragma unroll
+          for (int i = 0; i < kPW; ++i) {
+            const int pm = warp * kPer + i0 + i;
+            const int ba = xq[pm].best_a;
+            av[i] = pp[pm].done ? -1 : ((ba >= 0 && ba < K) ? ba : 0);
+            bp[i] = 0.0;
+          }
+          for (int k = lane; k < n; k += 32) {
+            float dv[kPW], yv[kPW];
+#pragma unroll
+            for (int i = 0; i < kPW; ++i) {
+              dv[i] = av[i] >= 0 ? __ldg(D + int64_t(av[i]) * n + k) : 0.0f;
+              yv[i] = av[i] >= 0 ? __ldg(Y + (p0 + warp * kPer + i0 + i) * n + k) : 0.0f;
+            }
+#pragma unroll
+            for (int i = 0; i < kPW; ++i) bp[i] = fma(double(dv[i]), double(yv[i]), bp[i]);
+          }
+#pragma unroll
+          for (int i = 0; i < kPW; ++i) {
+            const double t = warp_sum(bp[i]);
+            if (lane == 0) xq[warp * kPer + i0 + i].best_b = t;
+          }
         }
       }
       __syncthreads();
@@ -576,6 +700,17 @@ __global__ void __launch_bounds__(kTbThreads, 1)
                 if (kc * 8 + e < n) r[e] = fmaf(-gg, __ldg(dr + e), r[e]);
             }
           }
+          if constexpr (F32) {
+            float* dst = Rt + size_t(m) * n + kc * 8;
+            if (d_vec4 && kc * 8 + 8 <= n) {
+              __stcg(reinterpret_cast<float4*>(dst), make_float4(r[0], r[1], r[2], r[3]));
+              __stcg(reinterpret_cast<float4*>(dst) + 1, make_float4(r[4], r[5], r[6], r[7]));
+            } else {
+#pragma unroll
+              for (int e = 0; e < 8; ++e)
+                if (kc * 8 + e < n) __stcg(dst + e, r[e]);
+            }
+          }
           if (fin) {
             float* dst = R_out + (p0 + m) * int64_t(n) + kc * 8;
             if (r_vec4 && kc * 8 + 8 <= n) {
@@ -608,6 +743,7 @@ __global__ void __launch_bounds__(kTbThreads, 1)
           tc += X.part[j].y;
         }
         P.rnorm = sqrtf(tc);
+        if constexpr (F32) P.rnorm = dmax * (TbOp<F16>::err * P.rnorm + slack * sqrtf(tn));
         if (sqrtf(tn) < 1e-3f) P.done = 1;
       }
     }
@@ -655,13 +791,17 @@ bool omp_tcb_supported(int n, int K, int L) {
          omp_tcb_smem_bytes(n, K, L) <= 232448 - 1024;
 }
 
-size_t omp_tcb_scratch_bytes(int n, int K) {
+// Scratch: the 16-bit dictionary | atom sums | F32: [4] words (the largest norm) |
+// F32: the residual rows of a tile per SM.
+size_t omp_tcb_scratch_bytes(int n, int K, TcForm form, int num_sms) {
   const TbLayout o = tb_layout(n, K, 1);
-  return size_t(o.Kp) * o.np16 * 2 + size_t(o.Kp) * 4;
+  size_t b = size_t(o.Kp) * o.np16 * 2 + size_t(o.Kp) * 4;
+  if (form == TcForm::kFp32) b += 16 + size_t(num_sms) * kTbTile * n * 4;
+  return b;
 }
 
 cudaError_t launch_omp_tcb(const float* patches, int64_t N, int n, const float* dict, const double* gram, int K,
-                           int L, int32_t* idx, float* coef, int num_sms, int fp16, void* scratch,
+                           int L, int32_t* idx, float* coef, int num_sms, TcForm form, void* scratch,
                            GridBarrier* flags, DevStats* stats, cudaStream_t s, float* resid_out, int* last_out,
                            int64_t* fix_list, unsigned long long* fix_count) {
   if (!omp_tcb_supported(n, K, L)) return cudaErrorInvalidValue;
@@ -669,14 +809,25 @@ cudaError_t launch_omp_tcb(const float* patches, int64_t N, int n, const float* 
   const TbLayout o = tb_layout(n, K, L);
   unsigned char* Bg = static_cast<unsigned char*>(scratch);
   float* asum = reinterpret_cast<float*>(Bg + size_t(o.Kp) * o.np16 * 2);
-  if (fp16)
-    tb_prep_kernel<true><<<num_sms, 256, 0, s>>>(dict, K, n, o.Kp, o.np16, Bg, asum);
+  unsigned* sq_max = nullptr;
+  float* rg = nullptr;
+  cudaError_t e;
+  if (form == TcForm::kFp32) {
+    sq_max = reinterpret_cast<unsigned*>(asum + o.Kp);
+    rg = reinterpret_cast<float*>(sq_max + 4);
+    if ((e = cudaMemsetAsync(sq_max, 0, 16, s)) != cudaSuccess) return e;
+    tb_norm_kernel<<<(K + 7) / 8, 256, 0, s>>>(dict, K, n, sq_max);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  }
+  if (form != TcForm::kBf16)
+    tb_prep_kernel<true><<<num_sms, 256, 0, s>>>(dict, K, n, o.Kp, o.np16, Bg, asum, sq_max);
   else
-    tb_prep_kernel<false><<<num_sms, 256, 0, s>>>(dict, K, n, o.Kp, o.np16, Bg, asum);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
+    tb_prep_kernel<false><<<num_sms, 256, 0, s>>>(dict, K, n, o.Kp, o.np16, Bg, asum, sq_max);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
   const size_t smem = o.total;
-  auto kern = fp16 ? omp_tcb_kernel<true> : omp_tcb_kernel<false>;
+  auto kern = form == TcForm::kFp32  ? omp_tcb_kernel<true, true>
+              : form == TcForm::kFp16 ? omp_tcb_kernel<true, false>
+                                      : omp_tcb_kernel<false, false>;
   e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
   if (e != cudaSuccess) return e;
   const int64_t ntiles = (N + kTbTile - 1) / kTbTile;
@@ -687,7 +838,7 @@ cudaError_t launch_omp_tcb(const float* patches, int64_t N, int n, const float* 
                          : 0;
   const int r_vec4 = ((n & 3) == 0 && (reinterpret_cast<uintptr_t>(resid_out) & 15) == 0) ? 1 : 0;
   kern<<<grid, kTbThreads, smem, s>>>(patches, N, n, dict, Bg, asum, gram, K, L, idx, coef, ntiles, d_vec4,
-                                      resid_out, last_out, fix_list, fix_count, r_vec4, flags, stats);
+                                      resid_out, last_out, fix_list, fix_count, r_vec4, sq_max, rg, flags, stats);
   return cudaGetLastError();
 }
 

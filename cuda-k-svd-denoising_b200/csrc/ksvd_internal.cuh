@@ -84,6 +84,10 @@ bool omp_stream_supported(int n, int K, int L);
 cudaError_t launch_omp_stream(const float* patches, int64_t N, int n, const float* dict, const double* gram, int K,
                               int L, int32_t* idx, float* coef, int num_sms, DevStats* stats, cudaStream_t s);
 
+// The arithmetic form of a tensor-core OMP: 16-bit correlation with the exact
+// (FP64) argmax, or the FP32 argmax found through the FP16 correlation.
+enum class TcForm { kBf16, kFp16, kFp32 };
+
 // OMP with the BF16 tensor-core correlation and exact FP32/FP64 re-scoring.
 size_t omp_tc_smem_bytes(int n, int K, int L);
 bool omp_tc_supported(int n, int K, int L);
@@ -93,7 +97,7 @@ bool omp_tc_supported(int n, int K, int L);
 // caller) for launch_residual's list form.  last_out (with resid_out, N): the
 // highest support atom with a nonzero coefficient (-1 if none).
 cudaError_t launch_omp_tc(const float* patches, int64_t N, int n, const float* dict, const double* gram, int K,
-                          int L, int32_t* idx, float* coef, int num_sms, int fp16, GridBarrier* flags,
+                          int L, int32_t* idx, float* coef, int num_sms, TcForm form, GridBarrier* flags,
                           DevStats* stats, cudaStream_t s, float* resid_out = nullptr, int* last_out = nullptr,
                           int64_t* fix_list = nullptr, unsigned long long* fix_count = nullptr);
 
@@ -101,10 +105,10 @@ cudaError_t launch_omp_tc(const float* patches, int64_t N, int n, const float* d
 // resident kernel (atoms <= 512, n <= 256): the 16-bit dictionary streams
 // from `scratch` (omp_tcb_scratch_bytes, written by the launch).
 bool omp_tcb_supported(int n, int K, int L);
-size_t omp_tcb_scratch_bytes(int n, int K);
+size_t omp_tcb_scratch_bytes(int n, int K, TcForm form, int num_sms);
 // resid_out, last_out, fix_list, fix_count (optional): as for launch_omp_tc.
 cudaError_t launch_omp_tcb(const float* patches, int64_t N, int n, const float* dict, const double* gram, int K,
-                           int L, int32_t* idx, float* coef, int num_sms, int fp16, void* scratch,
+                           int L, int32_t* idx, float* coef, int num_sms, TcForm form, void* scratch,
                            GridBarrier* flags, DevStats* stats, cudaStream_t s, float* resid_out = nullptr,
                            int* last_out = nullptr, int64_t* fix_list = nullptr,
                            unsigned long long* fix_count = nullptr);

@@ -422,7 +422,8 @@ ksvd_status omp_learned_impl(ksvd_ctx* c, const float* d_patches, int64_t N, con
   KSVD_CU(c, ksvd::launch_gather_rows(d_patches, n, fb_list, m, fy, c->stream), "fallback gather");
   if (ksvd::omp_tc_supported(n, K, L)) {
     KSVD_CU(c,
-            ksvd::launch_omp_tc(fy, m, n, d_dict, gram, K, L, fi, fc, c->num_sms, 0, c->d_flags, nullptr, c->stream),
+            ksvd::launch_omp_tc(fy, m, n, d_dict, gram, K, L, fi, fc, c->num_sms, ksvd::TcForm::kBf16,
+                                c->d_flags, nullptr, c->stream),
             "fallback omp");
   } else {
     KSVD_CU(c, ksvd::launch_omp_fp32(fy, m, n, d_dict, gram, K, L, fi, fc, c->num_sms, nullptr, c->stream),

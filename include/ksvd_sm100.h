@@ -234,7 +234,7 @@ ksvd_status ksvd_profile_phases(ksvd_ctx* ctx, double* ms_out, int count);
  * Synchronises the stream. */
 ksvd_status ksvd_profile_counters(ksvd_ctx* ctx, int64_t* out, int count);
 
-/* OMP sparse coding (the same FP32 kernels and results as ksvd_omp) for
+/* OMP sparse coding (the FP32 kernels, the codes of ksvd_omp's FP32 form) for
  * callers that cannot allocate device memory: code inside a CUDA graph being
  * captured or replayed, plugins whose host framework owns every device
  * allocation, real-time loops that must not allocate once running.  It needs
