@@ -286,9 +286,9 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   const bool y_vec4 = (n & 3) == 0 && (reinterpret_cast<uintptr_t>(Y) & 15) == 0;
   int nscored = 0;
   int64_t p0 = 0;  // first patch of the current tile
-  // chunk kc of patch m's residual row into R_out
-  auto store_row_chunk = [&](int kc, const float (&r)[8]) {
-    float* dst = R_out + (p0 + m) * int64_t(n) + kc * 8;
+  // chunk kc of patch pm's residual row into R_out
+  auto store_row_chunk = [&](int pm, int kc, const float (&r)[8]) {
+    float* dst = R_out + (p0 + pm) * int64_t(n) + kc * 8;
     if (r_vec4 && kc * 8 + 8 <= n) {
       __stcg(reinterpret_cast<float4*>(dst), make_float4(r[0], r[1], r[2], r[3]));
       __stcg(reinterpret_cast<float4*>(dst) + 1, make_float4(r[4], r[5], r[6], r[7]));
@@ -667,21 +667,26 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       lap(12);
       // ---- residual quarter (FP32), partial norms, next A operand -----------
       // (with the patch's final coefficients, the row also goes to R_out)
-      const bool live = !done && !P.done;
+      // A patch's four threads are neighbouring lanes here and take its chunks in
+      // turn, so that a warp's load touches the lines of 8 rows, not of 32.
+      const int pm = warp * (kTcTile / (kTcThreads / 32)) + (lane >> 2), pc = lane & 3;
+      const TcPatch& RP = pp[pm];
+      const float* const pyr = Ys + pm * ysn;
+      const bool live = !RP.done;
       float nrm = 0.0f, cn = 0.0f;
       if (live) {
-        const int cnt = P.cnt;
+        const int cnt = RP.cnt;
         const bool fin = R_out != nullptr && cnt == L;
-        const float mean = P.rmean, inv = 1.0f / P.rscale;
-        for (int kc = kc_lo; kc < kc_hi; ++kc) {
+        const float mean = RP.rmean, inv = 1.0f / RP.rscale;
+        for (int kc = pc; kc < nkc; kc += kTcQ) {
           float r[8];
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
             const int kk = kc * 8 + e;
-            r[e] = (!F32 && kk < n) ? yr[kk] : 0.0f;
+            r[e] = (!F32 && kk < n) ? pyr[kk] : 0.0f;
           }
           if constexpr (F32) {  // the patch again, from L2
-            const float* yg = Y + (p0 + m) * n + kc * 8;
+            const float* yg = Y + (p0 + pm) * n + kc * 8;
             if (y_vec4 && kc * 8 + 8 <= n) {
               const float4 y0 = __ldg(reinterpret_cast<const float4*>(yg));
               const float4 y1 = __ldg(reinterpret_cast<const float4*>(yg) + 1);
@@ -702,8 +707,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
               for (int u = 0; u < kSB; ++u) {
                 const int s2 = s0 + u;
                 if (s2 < cnt) {
-                  const float4* dr = reinterpret_cast<const float4*>(D + int64_t(Ss[m * L + s2]) * n + kc * 8);
-                  gg[u] = gam[m * L + s2];
+                  const float4* dr = reinterpret_cast<const float4*>(D + int64_t(Ss[pm * L + s2]) * n + kc * 8);
+                  gg[u] = gam[pm * L + s2];
                   da[u] = __ldg(dr);
                   db[u] = __ldg(dr + 1);
                 }
@@ -724,18 +729,18 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             }
           } else {
             for (int s2 = 0; s2 < cnt; ++s2) {
-              const float gg = gam[m * L + s2];
-              const float* dr = D + int64_t(Ss[m * L + s2]) * n + kc * 8;
+              const float gg = gam[pm * L + s2];
+              const float* dr = D + int64_t(Ss[pm * L + s2]) * n + kc * 8;
 #pragma unroll
               for (int e = 0; e < 8; ++e)
                 if (kc * 8 + e < n) r[e] = fmaf(-gg, __ldg(dr + e), r[e]);
             }
           }
-          if (fin) store_row_chunk(kc, r);
+          if (fin) store_row_chunk(pm, kc, r);
           if constexpr (F32)
 #pragma unroll
             for (int e = 0; e < 8; ++e)
-              if (kc * 8 + e < n) Ys[m * ysn + kc * 8 + e] = r[e];
+              if (kc * 8 + e < n) Ys[pm * ysn + kc * 8 + e] = r[e];
           unsigned short h[8];
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
@@ -745,17 +750,16 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             cn = fmaf(c, c, cn);
             h[e] = Op16<F16>::cvt(c * inv);
           }
-          store8(At + canon_off(m, kc * 8, kTcTile), h);
+          store8(At + canon_off(pm, kc * 8, kTcTile), h);
         }
       }
-      float2* part = X.part;
-      part[q] = make_float2(nrm, cn);
+      xq[pm].part[pc] = make_float2(nrm, cn);
       __syncthreads();
-      if (q == 0 && live) {
+      if (q == 0 && !P.done) {
         float tn = 0.0f, tc = 0.0f;
         for (int j = 0; j < kTcQ; ++j) {
-          tn += part[j].x;
-          tc += part[j].y;
+          tn += X.part[j].x;
+          tc += X.part[j].y;
         }
         P.rnorm = sqrtf(tc);
         if constexpr (F32) P.rnorm = dmax * (Op16<F16>::err * P.rnorm + slack * sqrtf(tn));

@@ -268,7 +268,6 @@ __global__ void __launch_bounds__(kTbThreads, 1)
   const int m = g * 32 + lane;
   const unsigned lane_addr = tmem + (unsigned(g * 32) << 16);
   const int c_lo = q * qw, c_hi = min(Kp, c_lo + qw);
-  const int kc_lo = (nkc * q) / kTbQ, kc_hi = (nkc * (q + 1)) / kTbQ;
   TbPatch& P = pp[m];
   TbX& X = xq[m];
   double* Lp = Lc + m * tri;
@@ -331,33 +330,60 @@ __global__ void __launch_bounds__(kTbThreads, 1)
   for (int64_t tile = blockIdx.x; tile < ntiles && !failed; tile += gridDim.x) {
     const int64_t p0 = tile * kTbTile;
     const int np = (N - p0 < kTbTile) ? int(N - p0) : kTbTile;
-    const float* yg = Y + (p0 + (m < np ? m : 0)) * n;  // this patch's values (global)
-    // per-patch sums over a quarter of the features
+    // per-patch sums, norms and the first A operand: a patch's four threads are
+    // neighbouring lanes and take its 8-value chunks in turn (as in the residual)
+    const int sm = warp * (kTbTile / (kTbThreads / 32)) + (lane >> 2), sc = lane & 3;
+    const float* const yg = Y + (p0 + (sm < np ? sm : 0)) * n;
+    auto load_chunk = [&](int kc, float (&v)[8]) {
+      if (d_vec4 && kc * 8 + 8 <= n) {
+        const float4 y0 = __ldg(reinterpret_cast<const float4*>(yg + kc * 8));
+        const float4 y1 = __ldg(reinterpret_cast<const float4*>(yg + kc * 8) + 1);
+        v[0] = y0.x, v[1] = y0.y, v[2] = y0.z, v[3] = y0.w;
+        v[4] = y1.x, v[5] = y1.y, v[6] = y1.z, v[7] = y1.w;
+      } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = (kc * 8 + e < n) ? __ldg(yg + kc * 8 + e) : 0.0f;
+      }
+    };
     {
       float ys = 0.0f;
       double yy = 0.0;
-      if (m < np)
-        for (int k = q; k < n; k += kTbQ) {
-          const float v = __ldg(yg + k);
-          ys += v;
-          yy = fma(double(v), double(v), yy);
+      if (sm < np)
+        for (int kc = sc; kc < nkc; kc += kTbQ) {
+          float v[8];
+          load_chunk(kc, v);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {  // zeros beyond n
+            ys += v[e];
+            yy = fma(double(v[e]), double(v[e]), yy);
+          }
         }
-      X.part[q].x = ys;
-      X.qmask[q][0] = static_cast<unsigned long long>(__double_as_longlong(yy));
+      xq[sm].part[sc].x = ys;
+      xq[sm].qmask[sc][0] = static_cast<unsigned long long>(__double_as_longlong(yy));
     }
     __syncthreads();
     {
-      const float ys = (X.part[0].x + X.part[1].x) + (X.part[2].x + X.part[3].x);
+      const TbX& SX = xq[sm];
+      const float ys = (SX.part[0].x + SX.part[1].x) + (SX.part[2].x + SX.part[3].x);
       const float mean = ys / float(n);
       float mx = 0.0f, cc = 0.0f;
-      if (m < np)
-        for (int k = q; k < n; k += kTbQ) {
-          const float c = __ldg(yg + k) - mean;
-          mx = fmaxf(mx, fabsf(c));
-          cc = fmaf(c, c, cc);
+      if (sm < np)
+        for (int kc = sc; kc < nkc; kc += kTbQ) {
+          float v[8];
+          load_chunk(kc, v);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            const float c = kc * 8 + e < n ? v[e] - mean : 0.0f;
+            mx = fmaxf(mx, fabsf(c));
+            cc = fmaf(c, c, cc);
+          }
         }
       __syncthreads();
-      X.part[q] = make_float2(mx, cc);
+      xq[sm].part[sc] = make_float2(mx, cc);
+      if (sc == 0) {
+        pp[sm].ysum = ys;
+        pp[sm].rmean = mean;
+      }
       __syncthreads();
       if (q == 0) {
         double yy = 0.0;
@@ -365,9 +391,7 @@ __global__ void __launch_bounds__(kTbThreads, 1)
         for (int j = 0; j < kTbQ; ++j) yy += __longlong_as_double(static_cast<long long>(X.qmask[j][0]));
         P.cnt = 0;
         P.done = m >= np;
-        P.ysum = ys;
         P.yy = yy;
-        P.rmean = mean;
         P.rscale = tb_pow2_scale(fmaxf(fmaxf(X.part[0].x, X.part[1].x), fmaxf(X.part[2].x, X.part[3].x)));
         P.rnorm = sqrtf((X.part[0].y + X.part[1].y) + (X.part[2].y + X.part[3].y));
         if constexpr (F32) P.rnorm = dmax * (TbOp<F16>::err * P.rnorm + slack * sqrtf(float(yy)));
@@ -375,15 +399,15 @@ __global__ void __launch_bounds__(kTbThreads, 1)
     }
     __syncthreads();
     {
-      const float mean = P.rmean, inv = 1.0f / P.rscale;
-      for (int kc = kc_lo; kc < kc_hi; ++kc) {
+      const float mean = pp[sm].rmean, inv = 1.0f / pp[sm].rscale;
+      for (int kc = sc; kc < nkc; kc += kTbQ) {
+        float v[8];
+        load_chunk(kc, v);
         unsigned short h[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const int k = kc * 8 + e;
-          h[e] = TbOp<F16>::cvt((k < n && m < np) ? (__ldg(yg + k) - mean) * inv : 0.0f);
-        }
-        tb_store8(At + canon_off(m, kc * 8, kTbTile), h);
+        for (int e = 0; e < 8; ++e)
+          h[e] = TbOp<F16>::cvt((kc * 8 + e < n && sm < np) ? (v[e] - mean) * inv : 0.0f);
+        tb_store8(At + canon_off(sm, kc * 8, kTbTile), h);
       }
     }
     for (int step = 0; step < L; ++step) {
@@ -660,22 +684,27 @@ __global__ void __launch_bounds__(kTbThreads, 1)
       __syncthreads();
       // ---- residual quarter (FP32), partial norms, next A operand -----------
       // (with the patch's final coefficients, the row also goes to R_out)
-      const bool live = !done && !P.done;
+      // A patch's four threads are neighbouring lanes here and take its chunks in
+      // turn, so that a warp's load touches the lines of 8 rows, not of 32.
+      const int pm = warp * (kTbTile / (kTbThreads / 32)) + (lane >> 2), pc = lane & 3;
+      const TbPatch& RP = pp[pm];
+      const float* const pyg = Y + (p0 + pm) * n;
+      const bool live = !RP.done;
       float nrm = 0.0f, cn = 0.0f;
       if (live) {
-        const int cnt = P.cnt;
+        const int cnt = RP.cnt;
         const bool fin = R_out != nullptr && cnt == L;
-        const float mean = P.rmean, inv = 1.0f / P.rscale;
-        for (int kc = kc_lo; kc < kc_hi; ++kc) {
+        const float mean = RP.rmean, inv = 1.0f / RP.rscale;
+        for (int kc = pc; kc < nkc; kc += kTbQ) {
           float r[8];
           if (d_vec4 && kc * 8 + 8 <= n) {
-            const float4 y0 = __ldg(reinterpret_cast<const float4*>(yg + kc * 8));
-            const float4 y1 = __ldg(reinterpret_cast<const float4*>(yg + kc * 8) + 1);
+            const float4 y0 = __ldg(reinterpret_cast<const float4*>(pyg + kc * 8));
+            const float4 y1 = __ldg(reinterpret_cast<const float4*>(pyg + kc * 8) + 1);
             r[0] = y0.x, r[1] = y0.y, r[2] = y0.z, r[3] = y0.w;
             r[4] = y1.x, r[5] = y1.y, r[6] = y1.z, r[7] = y1.w;
             for (int s2 = 0; s2 < cnt; ++s2) {
-              const float4* dr = reinterpret_cast<const float4*>(D + int64_t(Ss[m * L + s2]) * n + kc * 8);
-              const float gg = gam[m * L + s2];
+              const float4* dr = reinterpret_cast<const float4*>(D + int64_t(Ss[pm * L + s2]) * n + kc * 8);
+              const float gg = gam[pm * L + s2];
               const float4 da = __ldg(dr), db = __ldg(dr + 1);
               r[0] = fmaf(-gg, da.x, r[0]);
               r[1] = fmaf(-gg, da.y, r[1]);
@@ -690,18 +719,18 @@ __global__ void __launch_bounds__(kTbThreads, 1)
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
               const int kk = kc * 8 + e;
-              r[e] = (kk < n) ? __ldg(yg + kk) : 0.0f;
+              r[e] = (kk < n) ? __ldg(pyg + kk) : 0.0f;
             }
             for (int s2 = 0; s2 < cnt; ++s2) {
-              const float gg = gam[m * L + s2];
-              const float* dr = D + int64_t(Ss[m * L + s2]) * n + kc * 8;
+              const float gg = gam[pm * L + s2];
+              const float* dr = D + int64_t(Ss[pm * L + s2]) * n + kc * 8;
 #pragma unroll
               for (int e = 0; e < 8; ++e)
                 if (kc * 8 + e < n) r[e] = fmaf(-gg, __ldg(dr + e), r[e]);
             }
           }
           if constexpr (F32) {
-            float* dst = Rt + size_t(m) * n + kc * 8;
+            float* dst = Rt + size_t(pm) * n + kc * 8;
             if (d_vec4 && kc * 8 + 8 <= n) {
               __stcg(reinterpret_cast<float4*>(dst), make_float4(r[0], r[1], r[2], r[3]));
               __stcg(reinterpret_cast<float4*>(dst) + 1, make_float4(r[4], r[5], r[6], r[7]));
@@ -712,7 +741,7 @@ __global__ void __launch_bounds__(kTbThreads, 1)
             }
           }
           if (fin) {
-            float* dst = R_out + (p0 + m) * int64_t(n) + kc * 8;
+            float* dst = R_out + (p0 + pm) * int64_t(n) + kc * 8;
             if (r_vec4 && kc * 8 + 8 <= n) {
               __stcg(reinterpret_cast<float4*>(dst), make_float4(r[0], r[1], r[2], r[3]));
               __stcg(reinterpret_cast<float4*>(dst) + 1, make_float4(r[4], r[5], r[6], r[7]));
@@ -731,12 +760,12 @@ __global__ void __launch_bounds__(kTbThreads, 1)
             cn = fmaf(c, c, cn);
             h[e] = TbOp<F16>::cvt(c * inv);
           }
-          tb_store8(At + canon_off(m, kc * 8, kTbTile), h);
+          tb_store8(At + canon_off(pm, kc * 8, kTbTile), h);
         }
       }
-      X.part[q] = make_float2(nrm, cn);
+      xq[pm].part[pc] = make_float2(nrm, cn);
       __syncthreads();
-      if (q == 0 && live) {
+      if (q == 0 && !P.done) {
         float tn = 0.0f, tc = 0.0f;
         for (int j = 0; j < kTbQ; ++j) {
           tn += X.part[j].x;
