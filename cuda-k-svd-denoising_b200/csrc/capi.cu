@@ -303,8 +303,8 @@ ksvd_status omp_form(ksvd_ctx* c, const float* d_patches, int64_t N, const float
   ksvd::DevStats* ph = c->profiling >= 2 ? c->d_phase : nullptr;
   // Every form runs on the tensor cores, with the 16-bit dictionary in shared
   // memory where it fits (up to 256 atoms), else streamed (up to 512 atoms);
-  // beyond that (and beyond 16 atoms per patch) the FP32 kernels run: the
-  // resident-dictionary one when it fits, else the streamed one.
+  // beyond that, beyond 16 atoms per patch and for few patches (below) the FP32
+  // kernels run: the resident-dictionary one when it fits, else the streamed one.
   // Before an update sweep the tensor-core kernels also write the sweep's residual
   // rows (the same buffers and arithmetic as launch_residual); patches that
   // took fewer than L atoms are listed and formed after them.
@@ -331,7 +331,16 @@ ksvd_status omp_form(ksvd_ctx* c, const float* d_patches, int64_t N, const float
   const ksvd::TcForm form = precision == KSVD_PREC_FP32           ? ksvd::TcForm::kFp32
                             : precision == KSVD_PREC_FP16_RESCORE ? ksvd::TcForm::kFp16
                                                                   : ksvd::TcForm::kBf16;
-  if (ksvd::omp_tc_supported(n, K, L)) {
+  // The FP32 kernel of small dictionaries works on tiles of 32 patches, the
+  // tensor-core ones on tiles of 128: where one or two waves of the former cover
+  // the patches it is the faster one (8 x 8 patches, 256 atoms: 54 us a wave
+  // against 107; 16 x 16: 209 against 272 with the dictionary streamed; with 512
+  // atoms a wave takes 549 against 494, so the tensor cores always win).
+  const int64_t simt_waves = (N + int64_t(32) * c->num_sms - 1) / (int64_t(32) * c->num_sms);
+  const bool simt = form == ksvd::TcForm::kFp32 && K <= 256 &&
+                    simt_waves <= (ksvd::omp_tc_supported(n, K, L) ? 2 : 1) &&
+                    (ksvd::omp_fp32_supported(n, K, L) || ksvd::omp_stream_supported(n, K, L));
+  if (!simt && ksvd::omp_tc_supported(n, K, L)) {
     if (for_update) KSVD_TRY(fused_buffers());
     KSVD_CU(c,
             ksvd::launch_omp_tc(d_patches, N, n, d_dict, gram, K, L, d_idx, d_coef, c->num_sms,
@@ -339,7 +348,7 @@ ksvd_status omp_form(ksvd_ctx* c, const float* d_patches, int64_t N, const float
                                 fix, nfix),
             "omp (tensor cores)");
     if (for_update) KSVD_TRY(listed_rows());
-  } else if (ksvd::omp_tcb_supported(n, K, L)) {
+  } else if (!simt && ksvd::omp_tcb_supported(n, K, L)) {
     void* scratch = nullptr;
     KSVD_TRY(ws(c, "tcb_scratch", ksvd::omp_tcb_scratch_bytes(n, K, form, c->num_sms), &scratch));
     if (for_update) KSVD_TRY(fused_buffers());

@@ -17,15 +17,17 @@
 // back as y (the reference would divide 0/0 there).
 #include <cuda_runtime.h>
 
+#include <cmath>
+
 #include "device_util.cuh"
 #include "ksvd_internal.cuh"
 
 namespace ksvd {
 
 // Two CTAs of 1024 threads per SM.  (2048 x 2048 image, 12 x 12 patches at stride 3:
-// 0.57 ms with a 32 x 16 tile, 0.80 with the square 16 x 16 one and 256 threads;
-// 48 x 32 tiles of one CTA per SM take 0.52 there, but lose where a tile of
-// larger patches has few pixels.)
+// 0.57 ms a rebuild with 32 x 16 tiles, 0.80 with square 16 x 16 ones and 256
+// threads; 48 x 32 tiles of one CTA per SM take 0.52 there, but lose where a
+// tile of larger patches has few pixels.)
 constexpr size_t kCol2imSmemLimit = 110 * 1024;
 constexpr int kCol2imThreads = 1024;
 
@@ -40,22 +42,28 @@ static size_t tile_bytes(const PatchGeom& g, Tile t) {
 }
 
 // Pixel tile of the shared-memory gather: of those whose covering patches fit
-// the budget, the one that forms the fewest patches per pixel (each patch is
-// formed once per tile it touches); x = 0 when none fits (large patches), in
-// which case the direct gather runs.
+// the budget, the one of the least modelled time, waves of CTAs x (rounds of
+// patches per warp + sums per pixel + set-up, in cycles).  Large tiles form
+// fewer patches per pixel (each patch is formed once per tile it touches);
+// small images and sparse patches want more CTAs.  x = 0 when no tile fits
+// (large patches), in which case the direct gather runs.
 static Tile pick_tile(const PatchGeom& g) {
   const int sides[] = {64, 48, 32, 24, 16, 8};
   Tile best{0, 0};
-  double cost = 0.0;
+  double least = 0.0;
   for (int tx : sides)
     for (int ty : sides) {
       const Tile t{tx, ty};
-      const size_t b = tile_bytes(g, t);
-      if (b > kCol2imSmemLimit) continue;
-      const double c = double(b) / (double(tx) * ty);
-      if (best.x == 0 || c < cost) {
+      if (tile_bytes(g, t) > kCol2imSmemLimit) continue;
+      const int np = tile_patches_1d(tx, g.ph, g.sh) * tile_patches_1d(ty, g.pw, g.sw);
+      const int cover = ((g.ph + g.sh - 1) / g.sh) * ((g.pw + g.sw - 1) / g.sw);
+      const double tiles = double((g.W + tx - 1) / tx) * ((g.H + ty - 1) / ty);
+      const double cta = 1200.0 * ((np + 31) / 32) * ((g.n + 159) / 160) +
+                         30.0 * cover * ((tx * ty + kCol2imThreads - 1) / kCol2imThreads) + 1500.0;
+      const double c = std::ceil(tiles / 296.0) * cta;  // two CTAs on each of 148 SMs
+      if (best.x == 0 || c < least) {
         best = t;
-        cost = c;
+        least = c;
       }
     }
   return best;

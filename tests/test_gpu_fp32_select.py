@@ -10,8 +10,11 @@ pytestmark = pytest.mark.gpu
 
 
 def _inputs(oracle, synth, pw, ph, K, kind):
+    # more than two waves of the SIMT kernel's tiles of 32 patches on 148 SMs, a
+    # ragged number: what the tensor cores take
     img = synth.add_gaussian(synth.clean_image(80, 11), 20.0, 11)
     Y = oracle.extract_patches(img, pw, ph, 2, 2)
+    Y = np.concatenate([Y * np.float32(1.0 + 0.01 * i) for i in range(9500 // Y.shape[0] + 1)])[:9501]
     D = oracle.init_dictionary(Y, K, int_norm=True, dtype=np.float32)
     if kind == "small atoms":
         D *= np.float32(1e-3)
