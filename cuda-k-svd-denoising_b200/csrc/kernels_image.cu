@@ -251,7 +251,7 @@ cudaError_t launch_col2im(const float* noisy, const PatchGeom& g, const float* d
     return cudaGetLastError();
   }
   const size_t smem = tile_bytes(g, t);
-  if (smem > 48 * 1024) {
+  if (smem > 47 * 1024) {  // with the static part beyond the default limit of 48 KB
     cudaError_t e = cudaFuncSetAttribute(col2im_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     if (e != cudaSuccess) return e;
   }

@@ -10,6 +10,8 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("pw,ph,sw,sh,w,h", [
     (3, 3, 3, 3, 70, 131),    # 64 x 64 tiles, the last ones partial
     (8, 8, 2, 2, 65, 64),
+    (8, 8, 2, 2, 128, 128),
+    (8, 8, 2, 2, 200, 200),   # tiles of exactly 48 KB among the candidates
     (12, 12, 3, 3, 100, 90),  # 32 x 16 tiles, uncovered border
     (6, 14, 4, 2, 90, 70),
     (16, 16, 2, 2, 60, 50),   # no tile fits
