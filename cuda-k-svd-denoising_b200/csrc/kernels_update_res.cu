@@ -527,7 +527,7 @@ __global__ void __launch_bounds__(kUrThreads, 1)
       if (jn < K && jn % kUrTab != 0) {
         const int4 ns = tab[jn % kUrTab];
         nact = ns.w;
-        prefetch = ns.y >= 0 && ns.y <= kUrThreads;
+        prefetch = ns.y >= 0 && min(ns.y, cap) <= kUrThreads;
         if (prefetch) {
           meta_entry(nm, ns.x, min(ns.y, cap), tid);
           nd = (tid < n) ? __ldcg(D + int64_t(jn) * n + tid) : 0.0f;
