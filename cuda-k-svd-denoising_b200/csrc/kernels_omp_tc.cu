@@ -35,6 +35,7 @@
 
 #include "device_util.cuh"
 #include "ksvd_internal.cuh"
+#include "omp_f32.cuh"
 #include "tcgen05_util.cuh"
 
 namespace ksvd {
@@ -149,10 +150,6 @@ __host__ __device__ inline TcLayout tc_layout(int n, int K, int L) {
   o.qw = int(tc_al((o.Kp + kTcQ - 1) / kTcQ, 16));  // columns per quarter, 16-column loads
   return o;
 }
-
-// F32: rounding of the FP32 sums (the scored one, the atom sums, the mean part)
-// per feature, in units of |r| |d|.
-constexpr float kF32Slack = 4.0f / 16777216.0f;
 
 template <bool F16, bool F32>
 __global__ void __launch_bounds__(kTcThreads, 1)
@@ -351,7 +348,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         P.rmean = mean;
         P.rscale = pow2_scale(fmaxf(fmaxf(X.part[0].x, X.part[1].x), fmaxf(X.part[2].x, X.part[3].x)));
         P.rnorm = sqrtf((X.part[0].y + X.part[1].y) + (X.part[2].y + X.part[3].y));
-        if constexpr (F32) P.rnorm = dmax * (Op16<F16>::err * P.rnorm + slack * sqrtf(float(yy)));
+        if constexpr (F32) P.rnorm = f32_bound(dmax, Op16<F16>::err, P.rnorm, slack, sqrtf(float(yy)));
       }
     }
     __syncthreads();
@@ -426,7 +423,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
           float gmax = X.qmax[0];
 #pragma unroll
           for (int j = 1; j < kTcQ; ++j) gmax = fmaxf(gmax, X.qmax[j]);
-          // (F32: rnorm is the whole error bound; where it is no number, all atoms)
+          // (F32: rnorm is the whole error bound; where it is infinite or no number, all atoms)
           const float thr = gmax - 2.0f * (F32 ? P.rnorm : Op16<F16>::err * P.rnorm);
 #pragma unroll
           for (int i = 0; i < 64; ++i) {
@@ -762,7 +759,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
           tc += X.part[j].y;
         }
         P.rnorm = sqrtf(tc);
-        if constexpr (F32) P.rnorm = dmax * (Op16<F16>::err * P.rnorm + slack * sqrtf(tn));
+        if constexpr (F32) P.rnorm = f32_bound(dmax, Op16<F16>::err, P.rnorm, slack, sqrtf(tn));
         if (sqrtf(tn) < 1e-3f) P.done = 1;
       }
       lap(9);

@@ -32,6 +32,7 @@
 
 #include "device_util.cuh"
 #include "ksvd_internal.cuh"
+#include "omp_f32.cuh"
 #include "tcgen05_util.cuh"
 
 namespace ksvd {
@@ -63,8 +64,6 @@ struct TbOp<true> {
   static constexpr unsigned fmt = 0u;
   static constexpr float err = kTbErrF16;
 };
-
-constexpr float kTbF32Slack = 4.0f / 16777216.0f;  // kF32Slack of kernels_omp_tc.cu
 
 __device__ __forceinline__ void tb_store8(unsigned char* dst, const unsigned short (&h)[8]) {
   uint4 v;
@@ -279,7 +278,7 @@ __global__ void __launch_bounds__(kTbThreads, 1)
     dmax = t.dmax;
     dscale = t.scale;
   }
-  const float slack = kTbF32Slack * float(n);
+  const float slack = kF32Slack * float(n);
   float* const Rt = F32 ? Rg + size_t(blockIdx.x) * kTbTile * n : nullptr;  // this tile's residual rows
 
   // thread 0: one step of MMAs over all K-slices, streaming the slices
@@ -394,7 +393,7 @@ __global__ void __launch_bounds__(kTbThreads, 1)
         P.yy = yy;
         P.rscale = tb_pow2_scale(fmaxf(fmaxf(X.part[0].x, X.part[1].x), fmaxf(X.part[2].x, X.part[3].x)));
         P.rnorm = sqrtf((X.part[0].y + X.part[1].y) + (X.part[2].y + X.part[3].y));
-        if constexpr (F32) P.rnorm = dmax * (TbOp<F16>::err * P.rnorm + slack * sqrtf(float(yy)));
+        if constexpr (F32) P.rnorm = f32_bound(dmax, TbOp<F16>::err, P.rnorm, slack, sqrtf(float(yy)));
       }
     }
     __syncthreads();
@@ -448,7 +447,7 @@ __global__ void __launch_bounds__(kTbThreads, 1)
         float gmax = X.qmax[0];
 #pragma unroll
         for (int j = 1; j < kTbQ; ++j) gmax = fmaxf(gmax, X.qmax[j]);
-        // (F32: rnorm is the whole error bound; where it is no number, all atoms)
+        // (F32: rnorm is the whole error bound; where it is infinite or no number, all atoms)
         const float thr = gmax - 2.0f * (F32 ? P.rnorm : TbOp<F16>::err * P.rnorm);
         for (int c0 = c_lo; c0 < c_hi; c0 += 16) {
           float v[16];
@@ -772,7 +771,7 @@ __global__ void __launch_bounds__(kTbThreads, 1)
           tc += X.part[j].y;
         }
         P.rnorm = sqrtf(tc);
-        if constexpr (F32) P.rnorm = dmax * (TbOp<F16>::err * P.rnorm + slack * sqrtf(tn));
+        if constexpr (F32) P.rnorm = f32_bound(dmax, TbOp<F16>::err, P.rnorm, slack, sqrtf(tn));
         if (sqrtf(tn) < 1e-3f) P.done = 1;
       }
     }

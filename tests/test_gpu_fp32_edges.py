@@ -1,0 +1,56 @@
+"""The FP32 OMP on the tensor cores against the FP32 SIMT kernels (which
+ksvd_omp_noalloc runs) where the window of atoms or the stop test is at its
+limits: the same codes, bit for bit."""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [
+    (8, 8, 200, 16),    # resident 16-bit dictionary
+    (5, 5, 16, 3),      # 25 values: no 16-byte rows
+    (8, 8, 257, 5),     # streamed 16-bit dictionary
+    (12, 12, 512, 5),   # the SIMT kernel streams too
+    (22, 21, 64, 5),    # 462 values
+]
+
+
+def _data(oracle, synth, pw, ph, K):
+    # more than two waves of the SIMT kernel's tiles of 32 patches on 148 SMs:
+    # what the tensor cores take
+    img = synth.add_gaussian(synth.clean_image(80, 11), 20.0, 11)
+    Y = oracle.extract_patches(img, pw, ph, 2, 2)
+    Y = np.concatenate([Y * np.float32(1.0 + 0.01 * i) for i in range(9500 // Y.shape[0] + 1)])[:9501]
+    return Y, oracle.init_dictionary(Y, K, int_norm=True, dtype=np.float32)
+
+
+def _both(torch, ksvd, pw, ph, L, Y, D):
+    params = ksvd.make_params(patch_width_dim=pw, patch_height_dim=ph, sliding_width=2, sliding_height=2,
+                              atoms=D.shape[0], omp_iter=L, precision=ksvd.PREC_FP32)
+    Yd, Dd = (torch.from_numpy(np.ascontiguousarray(a, dtype=np.float32)).cuda() for a in (Y, D))
+    codes = []
+    with ksvd.Context(params) as ctx:
+        for run in (ctx.omp, lambda *a: ksvd.omp_noalloc(params, *a)):
+            idx = torch.empty((Y.shape[0], L), dtype=torch.int32, device="cuda")
+            coef = torch.empty((Y.shape[0], L), device="cuda")
+            run(Yd, Dd, idx, coef)
+            torch.cuda.synchronize()
+            codes.append((idx.cpu().numpy(), coef.cpu().numpy()))
+    return codes
+
+
+def _assert_same(codes):
+    np.testing.assert_array_equal(codes[0][0], codes[1][0])
+    np.testing.assert_array_equal(codes[0][1], codes[1][1])
+
+
+@pytest.mark.parametrize("pw,ph,K,L", SHAPES)
+@pytest.mark.parametrize("scale", [1e-18, 1e-22, 1e-25, 1e-26, 1e-30, 1e-36])
+@pytest.mark.parametrize("centred", [False, True])
+def test_tiny_patches(torch_cuda, ksvd, oracle, synth, pw, ph, K, L, scale, centred):
+    """Patches whose squares leave the FP32 range."""
+    Y, D = _data(oracle, synth, pw, ph, K)
+    if centred:
+        Y = Y - Y.mean(1, keepdims=True)
+    _assert_same(_both(torch_cuda, ksvd, pw, ph, L, Y * np.float32(scale), D))
