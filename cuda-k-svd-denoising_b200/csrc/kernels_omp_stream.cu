@@ -248,11 +248,14 @@ __global__ void __launch_bounds__(kSThreads, 1)
         if (sqrtf(nrm) < 1e-3f) done[tid] = 1;
       }
       // ---- argmax per patch --------------------------------------------------
+      // (N > 0; with a -1 in sight the compiler takes |x| > -1 to hold for a NaN
+      // too, and an atom's NaN would beat every number)
+      const float none = N > 0 ? -1.0f : 0.0f;
       float bv[4];
       int bi[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        bv[j] = -1.0f;
+        bv[j] = none;
         bi[j] = 0x7fffffff;
       }
 #pragma unroll

@@ -54,3 +54,28 @@ def test_tiny_patches(torch_cuda, ksvd, oracle, synth, pw, ph, K, L, scale, cent
     if centred:
         Y = Y - Y.mean(1, keepdims=True)
     _assert_same(_both(torch_cuda, ksvd, pw, ph, L, Y * np.float32(scale), D))
+
+
+@pytest.mark.parametrize("pw,ph,K,L", SHAPES)
+def test_infinite_values(torch_cuda, ksvd, oracle, synth, pw, ph, K, L):
+    """Infinite values: an atom whose correlation is infinite is the largest, one
+    whose correlation is NaN is never chosen before a number (checked for the
+    first atom of a pursuit against the same sums in numpy)."""
+    Y, D = _data(oracle, synth, pw, ph, K)
+    D = D - D.mean(1, keepdims=True)
+    D /= np.linalg.norm(D, axis=1, keepdims=True)
+    D[7] = np.abs(D[7])  # one atom of one sign
+    D[0, 5] = 0.0        # infinity times zero
+    Y[:40] = np.inf
+    Y[40:80] = -np.inf
+    Y[80:120, 5] = np.inf
+    Y[120:160, 0] = np.inf
+    Y[120:160, 1] = -np.inf
+    Y[160:200, pw * ph - 1] = -np.inf
+    Y[200] = np.nan
+    codes = _both(torch_cuda, ksvd, pw, ph, L, Y, D)
+    _assert_same(codes)
+    with np.errstate(invalid="ignore"):
+        c = np.abs(np.add.reduce(D[None].astype(np.float64) * Y[:201, None].astype(np.float64), axis=2))
+    want = np.argmax(np.where(np.isnan(c), -1.0, c), axis=1)
+    np.testing.assert_array_equal(codes[0][0][:200, 0], want[:200])
