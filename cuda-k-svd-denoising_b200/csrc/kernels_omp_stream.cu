@@ -407,11 +407,14 @@ static void* s_fn(int apt) {
   }
 }
 
-bool omp_stream_supported(int n, int K, int L) {
+int omp_stream_chunk(int n, int K, int L) {
   const int apt = s_apt(K);
-  if (apt == 0 || L < 1 || L > kSLMax || n < 1) return false;
-  return omp_s_layout(n, apt, L).KC >= 4;
+  if (apt == 0 || L < 1 || L > kSLMax || n < 1) return 0;
+  const int kc = omp_s_layout(n, apt, L).KC;
+  return kc >= 4 ? kc : 0;
 }
+
+bool omp_stream_supported(int n, int K, int L) { return omp_stream_chunk(n, K, L) > 0; }
 
 cudaError_t launch_omp_stream(const float* patches, int64_t N, int n, const float* dict, const double* gram, int K,
                               int L, int32_t* idx, float* coef, int num_sms, DevStats* stats, cudaStream_t s) {

@@ -36,6 +36,7 @@
 #include "device_util.cuh"
 #include "ksvd_internal.cuh"
 #include "omp_f32.cuh"
+#include "omp_stop.cuh"
 #include "tcgen05_util.cuh"
 
 namespace ksvd {
@@ -157,7 +158,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                   const double* __restrict__ Gram, int K, int L, int32_t* __restrict__ idx_out,
                   float* __restrict__ coef_out, int64_t ntiles, int d_vec4, float* __restrict__ R_out,
                   int* __restrict__ last_out, int64_t* __restrict__ fix_list,
-                  unsigned long long* __restrict__ fix_count, int r_vec4, GridBarrier* flags, DevStats* stats) {
+                  unsigned long long* __restrict__ fix_count, int r_vec4, int stop_order, GridBarrier* flags,
+                  DevStats* stats) {
   extern __shared__ __align__(128) unsigned char smem[];
   const TcLayout lo = tc_layout(n, K, L);
   unsigned char* Bt = smem + lo.off_b;
@@ -760,6 +762,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         }
         P.rnorm = sqrtf(tc);
         if constexpr (F32) P.rnorm = f32_bound(dmax, Op16<F16>::err, P.rnorm, slack, sqrtf(tn));
+        if (stop_near(tn)) tn = stop_norm2(Y + (p0 + m) * n, D, n, Ss + m * L, gam + m * L, P.cnt, stop_order);
         if (sqrtf(tn) < 1e-3f) P.done = 1;
       }
       lap(9);
@@ -818,8 +821,9 @@ cudaError_t launch_omp_tc(const float* patches, int64_t N, int n, const float* d
   const int d_vec4 = ((n & 3) == 0 && (reinterpret_cast<uintptr_t>(dict) & 15) == 0) ? 1 : 0;
   const int r_vec4 = ((n & 3) == 0 && (reinterpret_cast<uintptr_t>(resid_out) & 15) == 0) ? 1 : 0;
   if (resid_out && (!last_out || !fix_list || !fix_count)) return cudaErrorInvalidValue;
+  const int stop_order = omp_stop_order(form, n, K, L);
   kern<<<grid, kTcThreads, smem, s>>>(patches, N, n, dict, gram, K, L, idx, coef, ntiles, d_vec4, resid_out, last_out,
-                                      fix_list, fix_count, r_vec4, flags, stats);
+                                      fix_list, fix_count, r_vec4, stop_order, flags, stats);
   return cudaGetLastError();
 }
 

@@ -33,6 +33,7 @@
 #include "device_util.cuh"
 #include "ksvd_internal.cuh"
 #include "omp_f32.cuh"
+#include "omp_stop.cuh"
 #include "tcgen05_util.cuh"
 
 namespace ksvd {
@@ -211,7 +212,7 @@ __global__ void __launch_bounds__(kTbThreads, 1)
                    float* __restrict__ coef_out, int64_t ntiles, int d_vec4, float* __restrict__ R_out,
                    int* __restrict__ last_out, int64_t* __restrict__ fix_list,
                    unsigned long long* __restrict__ fix_count, int r_vec4, const unsigned* __restrict__ sq_max,
-                   float* __restrict__ Rg, GridBarrier* flags, DevStats* stats) {
+                   float* __restrict__ Rg, int stop_order, GridBarrier* flags, DevStats* stats) {
   extern __shared__ __align__(128) unsigned char smem[];
   const TbLayout lo = tb_layout(n, K, L);
   unsigned char* ring = smem + lo.off_ring;
@@ -772,6 +773,7 @@ __global__ void __launch_bounds__(kTbThreads, 1)
         }
         P.rnorm = sqrtf(tc);
         if constexpr (F32) P.rnorm = f32_bound(dmax, TbOp<F16>::err, P.rnorm, slack, sqrtf(tn));
+        if (stop_near(tn)) tn = stop_norm2(Y + (p0 + m) * n, D, n, Ss + m * L, gam + m * L, P.cnt, stop_order);
         if (sqrtf(tn) < 1e-3f) P.done = 1;
       }
     }
@@ -865,8 +867,10 @@ cudaError_t launch_omp_tcb(const float* patches, int64_t N, int n, const float* 
                          ? 1
                          : 0;
   const int r_vec4 = ((n & 3) == 0 && (reinterpret_cast<uintptr_t>(resid_out) & 15) == 0) ? 1 : 0;
+  const int stop_order = omp_stop_order(form, n, K, L);
   kern<<<grid, kTbThreads, smem, s>>>(patches, N, n, dict, Bg, asum, gram, K, L, idx, coef, ntiles, d_vec4,
-                                      resid_out, last_out, fix_list, fix_count, r_vec4, sq_max, rg, flags, stats);
+                                      resid_out, last_out, fix_list, fix_count, r_vec4, sq_max, rg, stop_order,
+                                      flags, stats);
   return cudaGetLastError();
 }
 
