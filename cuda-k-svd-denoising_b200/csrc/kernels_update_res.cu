@@ -305,6 +305,9 @@ __global__ void __launch_bounds__(kUrThreads, 1)
   for (int gi = 0; gi < batch.ngroups; ++gi) {
     const UpdGroup& grp = batch.g[gi];
     if (int(blockIdx.x) < grp.cta_begin || int(blockIdx.x) >= grp.cta_begin + grp.ctas) continue;
+    // bulk copies of this group may land where the previous one, of another
+    // layout, kept its tables (fill_tab's barrier follows)
+    fence_proxy_async_smem();
     float* const R = grp.R;
     float* const D = grp.D;
     float* const coef = grp.coef;
