@@ -212,12 +212,17 @@ KSVD_DEV uint4 ld_word(const uint4* p) {
   return make_uint4(unsigned(lo), unsigned(lo >> 32), unsigned(hi), unsigned(hi >> 32));
 }
 
+// CTAs whose partials travel as words: at most this many a group of partials
+// (more go behind a counter, see `counted`).
+constexpr int kUrWordRounds = 2;
+
 // Sum of the words p[0], p[stride], ... (count of them) in ascending order, once
-// they show the tag: up to kB are polled together (re-reading one word after the
-// other would cost an L2 round trip each).  w of the result: 1, or 0 when the
-// time is over or an error is flagged elsewhere.
+// they show the tag: up to kUrWordRounds are polled together (re-reading one word
+// after the other would cost an L2 round trip each; eight at a time cost every
+// instantiation 12 to 50 bytes of spilled registers).  w of the result: 1, or 0
+// when the time is over or an error is flagged elsewhere.
 KSVD_DEV float4 ur_gather(const uint4* p, size_t stride, int count, unsigned tag, GridBarrier* flags) {
-  constexpr int kB = 8;
+  constexpr int kB = kUrWordRounds;
   float4 a = make_float4(0.f, 0.f, 0.f, 1.f);
   for (int i = 0; i < count; i += kB) {
     uint4 v[kB];
@@ -340,10 +345,14 @@ __global__ void __launch_bounds__(kUrThreads, 1)
     const int d_q = kUrThreads / F, d_f = kUrThreads - d_q * F;
     float4* const u4 = reinterpret_cast<float4*>(u);
     const float4* const wsum4 = reinterpret_cast<const float4*>(wsum);
+    // w pass: a warp per column group with its lanes over the features, or a
+    // float4 of a group per thread.  The former needs a group for most warps (n <=
+    // 224; with 8 groups, 512 x 512, 16 x 16, the local pass takes 2.1 ms a sweep
+    // against 1.3) and runs 32 NW features, NW of the launch's widest patch (the
+    // latter with 144 features: 1.3 ms at 2048 x 2048 against 1.1).
+    const bool lanes_w = 2 * Gr > kUrWarps && NW == (n + 31) / 32;
     // bulk copies need 16-byte aligned rows of a multiple of 16 bytes
     const bool tma = (n & 3) == 0 && (reinterpret_cast<uintptr_t>(R) & 15) == 0;
-    // w pass: the warp's column group and its share of the 32-feature chunks
-    const int H = kUrWarps / Gr, wg = warp % Gr, wh = warp / Gr;
 
     // this CTA's slice [sb, sb + m) of each of the next kUrTab atoms' c entries:
     // first entry, m (-1: no part in the atom), entries that enter the power
@@ -454,8 +463,11 @@ __global__ void __launch_bounds__(kUrThreads, 1)
       // polls, instead of as tagged words that every thread polls.  Tagged words
       // save a release and a round trip a step (1.8 against 2.1 us with 9 CTAs,
       // 144 features), but each carries a quarter more bytes and the polls of many
-      // CTAs slow the stores they wait for (3.2 against 3.0 us with 141 CTAs).
-      const bool counted = active > 2 * Gr;
+      // CTAs slow the stores they wait for (3.2 against 3.0 us with 141 CTAs).  In
+      // between it hardly matters: with the line at 1, 2, 3 or 4 words a group, sweeps
+      // with 3 to 61 CTAs an atom and 64 to 484 features differ by 1.5% at most
+      // (512 x 512, 16 x 16, 19 CTAs: 4.49, 4.48, 4.45, 4.46 ms).
+      const bool counted = active > kUrWordRounds * Gr;
       float* const v_s = xold_b + slot * cap;  // old coefficients, then per-column scalars
       const int* const row_s = row_b + slot * cap;
       const float* const dold = dbuf + slot * n4;
@@ -588,13 +600,9 @@ __global__ void __launch_bounds__(kUrThreads, 1)
           }
         }
         if (streamed) {  // columns beyond the capacity: a warp per two columns
-          float ur[NW], wacc[NW];
+          float wacc[NW];
 #pragma unroll
-          for (int k = 0; k < NW; ++k) {
-            const int i = lane + 32 * k;
-            ur[k] = (i < n) ? uc[i] : 0.0f;
-            wacc[k] = 0.0f;
-          }
+          for (int k = 0; k < NW; ++k) wacc[k] = 0.0f;
           for (int q = cap + warp; q < mc; q += 2 * kUrWarps) {
             float e0[NW], e1[NW];
             int ea, eb;
@@ -602,8 +610,9 @@ __global__ void __launch_bounds__(kUrThreads, 1)
             float d0 = 0.0f, d1 = 0.0f;
 #pragma unroll
             for (int k = 0; k < NW; ++k) {
-              d0 = fmaf(ur[k], e0[k], d0);
-              d1 = fmaf(ur[k], e1[k], d1);
+              const float w = lane + 32 * k < n ? uc[lane + 32 * k] : 0.0f;
+              d0 = fmaf(w, e0[k], d0);
+              d1 = fmaf(w, e1[k], d1);
             }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
@@ -620,9 +629,8 @@ __global__ void __launch_bounds__(kUrThreads, 1)
           }
         }
         __syncthreads();
-        // w = sum_q v_q e_q: the columns q = wg, wg + Gr, ... of a group, lanes
-        // over the features, the 32-feature chunks wh, wh + H, ...
-        if (H == 1) {
+        // w = sum_q v_q e_q: the columns q = g, g + Gr, ... of group g in order
+        if (lanes_w) {  // a warp per group, lanes over the features
           if (warp < Gr) {
             float acc[NW];
 #pragma unroll
@@ -639,22 +647,18 @@ __global__ void __launch_bounds__(kUrThreads, 1)
             for (int k = 0; k < NW; ++k)
               if (32 * k + lane < n4) wred[warp * n4 + 32 * k + lane] = acc[k];
           }
-        } else if (wh < H) {
-          constexpr int kC = 6;  // chunks of a warp (H grows as Gr falls)
-          float acc[kC];
-#pragma unroll
-          for (int k = 0; k < kC; ++k) acc[k] = 0.0f;
-#pragma unroll 2
-          for (int q = wg; q < mcr; q += Gr) {
+        } else if (s_q < Gr) {  // a float4 of a group per thread
+          float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+          for (int q = s_q; q < mcr; q += Gr) {
             const float v = v_s[q];
-            const float* const eq = Es + size_t(q) * es + 32 * wh + lane;
-#pragma unroll
-            for (int k = 0; k < kC; ++k)
-              if (32 * (wh + H * k) + lane < n4) acc[k] = fmaf(v, eq[32 * H * k], acc[k]);
+            const float4 e = Es4[q * es4 + s_f];
+            acc.x = fmaf(v, e.x, acc.x);
+            acc.y = fmaf(v, e.y, acc.y);
+            acc.z = fmaf(v, e.z, acc.z);
+            acc.w = fmaf(v, e.w, acc.w);
           }
-#pragma unroll
-          for (int k = 0; k < kC; ++k)
-            if (32 * (wh + H * k) + lane < n4) wred[wg * n4 + 32 * (wh + H * k) + lane] = acc[k];
+          reinterpret_cast<float4*>(wred)[s_q * F + s_f] = acc;
         }
         __syncthreads();
         lap(2);

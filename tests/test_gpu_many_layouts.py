@@ -35,3 +35,29 @@ def test_layouts_in_turn(torch_cuda, ksvd, synth):
         with ksvd.Context(params) as ctx:
             single, _ = ctx.denoise(noisy, s2)
         assert abs(synth.psnr(c, single) - synth.psnr(c, a)) <= 0.02
+
+
+# patch side, image side: 49 to 484 values, not all a multiple of four
+SMALL = [[(22, 64), (8, 40), (12, 48), (7, 39)], [(22, 64), (8, 44), (12, 50)]]
+
+
+@pytest.mark.parametrize("spec", SMALL)
+def test_small_plan_leaves_slices(ksvd, built_lib, spec):
+    """Every image of these batches has a CTA for each 64 of its patches, so its atoms are
+    cut into the same slices as on the whole GPU."""
+    _, ctas, _, _ = ksvd.many_plan([(_params(ksvd, p), s, s) for p, s in spec])
+    assert all(64 * c >= ((s - p) // 2 + 1) ** 2 for c, (p, s) in zip(ctas, spec))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("spec", SMALL)
+def test_mixed_batch_same_bits(torch_cuda, ksvd, synth, spec):
+    """The same slices, hence the same sums in the same order, whatever the widest
+    patch of the launch: the images of the batch equal the one-image path's."""
+    jobs = [(_params(ksvd, p), synth.add_gaussian(synth.clean_image(s, 90 + i), 20.0, 90 + i), 400.0)
+            for i, (p, s) in enumerate(spec)]
+    outs, _ = ksvd.denoise_many(jobs, tune=False)
+    for (params, noisy, s2), a in zip(jobs, outs):
+        with ksvd.Context(params) as ctx:
+            single, _ = ctx.denoise(noisy, s2)
+        np.testing.assert_array_equal(a, single)
