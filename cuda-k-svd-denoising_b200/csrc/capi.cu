@@ -517,14 +517,14 @@ ksvd_status ksvd_build_image(ksvd_ctx* c, const float* d_noisy, int width, int h
   double* partials = nullptr;
   double* lam = nullptr;
   KSVD_TRY(wsT(c, "img_acc", size_t(width) * height, &acc));
-  KSVD_TRY(wsT(c, "img_partials", size_t(ksvd::col2im_num_tiles(g)), &partials));
+  KSVD_TRY(wsT(c, "img_partials", size_t(ksvd::col2im_num_tiles(g, c->p.omp_iter, c->num_sms)), &partials));
   KSVD_TRY(wsT(c, "img_lambda", 1, &lam));
   int np = 0;
   {
     Prof pr(c, "col2im", 1);
     KSVD_CU(c,
             ksvd::launch_col2im(d_noisy, g, d_dict, c->p.atoms, c->p.omp_iter, d_idx, d_coef, acc, partials, &np,
-                                c->stream),
+                                c->num_sms, c->stream),
             "col2im");
   }
   {

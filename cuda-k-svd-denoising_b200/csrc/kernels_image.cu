@@ -2,9 +2,9 @@
 //
 // The reference forms all denoised patches D X with one SGEMM, copies them to
 // the host and overlap-adds them in a single host thread.  Here:
-//   col2im_kernel  one CTA per pixel tile (sides of 8 to 64; large
-//                  patches use col2im_direct_kernel, one thread per pixel,
-//                  with the same sums): the denoised patches that
+//   col2im_kernel  one CTA per pixel tile (sides of 8 to 64; where that is
+//                  slower, col2im_direct_kernel, one thread per pixel, with
+//                  the same sums): the denoised patches that
 //                  cover the tile (x_hat_p = sum_s x_s d_s from the compact
 //                  codes) are formed in shared memory, then each pixel sums
 //                  the covering patches in patch order (ix, then iy, the
@@ -17,6 +17,7 @@
 // back as y (the reference would divide 0/0 there).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 
 #include "device_util.cuh"
@@ -24,13 +25,16 @@
 
 namespace ksvd {
 
-// Two CTAs of 1024 threads per SM.  (2048 x 2048 image, 12 x 12 patches at stride 3:
-// 0.57 ms a rebuild with 32 x 16 tiles, 0.80 with square 16 x 16 ones and 256
-// threads; 48 x 32 tiles of one CTA per SM take 0.52 there, but lose where a
-// tile of larger patches has few pixels.)
-constexpr size_t kCol2imSmemLimit = 110 * 1024;
+// One CTA of 1024 threads per SM: its 63 registers a thread fill the register
+// file, so the tile may have nearly all of the shared memory.  (2048 x 2048
+// image, 12 x 12 patches at stride 3: 0.46 ms a rebuild with 64 x 32 tiles; with
+// 110 KB, 32 x 16 tiles, 0.52; two CTAs of 512 threads, 24 x 32 tiles, 0.50; four
+// of 256, 8 x 24 tiles, 0.78.)
+constexpr size_t kCol2imSmemLimit = 220 * 1024;
 constexpr int kCol2imThreads = 1024;
+constexpr int kDirectThreads = 256;
 
+static int ceil_div(int a, int b) { return (a + b - 1) / b; }
 static int tile_patches_1d(int TS, int ext, int stride) { return (TS + ext - 1) / stride + 1; }
 
 struct Tile {
@@ -41,40 +45,54 @@ static size_t tile_bytes(const PatchGeom& g, Tile t) {
   return size_t(tile_patches_1d(t.x, g.ph, g.sh)) * tile_patches_1d(t.y, g.pw, g.sw) * g.n * sizeof(float);
 }
 
-// Pixel tile of the shared-memory gather: of those whose covering patches fit
-// the budget, the one of the least modelled time, waves of CTAs x (rounds of
-// patches per warp + sums per pixel + set-up, in cycles).  Large tiles form
-// fewer patches per pixel (each patch is formed once per tile it touches);
-// small images and sparse patches want more CTAs.  x = 0 when no tile fits
-// (large patches), in which case the direct gather runs.
-static Tile pick_tile(const PatchGeom& g) {
+// Modelled time (us) of a rebuild with tile t: waves of one CTA per SM, each
+// forming its patches (rounds of a patch per warp, 160 features and 4 atoms at a
+// time, and their shared-memory stores) and summing its pixels.
+static double tile_us(const PatchGeom& g, int L, int num_sms, Tile t) {
+  const int np = std::min(tile_patches_1d(t.x, g.ph, g.sh), g.nx) * std::min(tile_patches_1d(t.y, g.pw, g.sw), g.ny);
+  const double waves = std::ceil(double(ceil_div(g.W, t.x)) * ceil_div(g.H, t.y) / num_sms);
+  const double rounds = ceil_div(np, kCol2imThreads / 32);
+  return 6.8 + waves * (rounds * (0.46 * ceil_div(g.n, 160) * ceil_div(L, 4) + 0.62) +
+                        1.33 * ceil_div(t.x * t.y, kCol2imThreads) + 0.75 + 2.1e-5 * np * g.n * L);
+}
+
+// The same of the gather without tiles: a thread per pixel forms the elements it
+// needs, lanes along x, so a warp's loads touch fewer lines with a larger step.
+static double direct_us(const PatchGeom& g, int L) {
+  const double sh = g.sh, cover = double(ceil_div(g.ph, g.sh)) * ceil_div(g.pw, g.sw);
+  return 11.6 + 1e-6 * g.W * g.H * cover * (2.73 + L * (0.82 / sh + 7.7 / (sh * sh) + 0.045 * g.pw));
+}
+
+// Pixel tile of the shared-memory gather, or x = 0 for the gather without tiles:
+// the one of the least modelled time.  Large tiles form fewer patches per pixel
+// (each patch is formed once per tile it touches), small images want more CTAs;
+// pixels that few patches cover, and patches of which few fit a tile, are faster
+// gathered.  The constants are a least-squares fit (8% for tiles, 18% for the
+// gather) to each tile's time on 20 geometries (patches of 4 x 4 to 22 x 22, steps
+// 1 to 8, 128 x 128 to 2048 x 2048); its choice is within 15% of the fastest tile on
+// all of them.  (2048 x 2048, 20 x 20 at stride 4: 2.92 ms with the largest tile in
+// 110 KB, 1.20 with 24 x 24; 8 x 8 at stride 4: 0.20 with tiles, 0.16 without.)
+static Tile pick_tile(const PatchGeom& g, int L, int num_sms) {
   const int sides[] = {64, 48, 32, 24, 16, 8};
   Tile best{0, 0};
-  double least = 0.0;
+  double least = direct_us(g, L);
   for (int tx : sides)
     for (int ty : sides) {
       const Tile t{tx, ty};
       if (tile_bytes(g, t) > kCol2imSmemLimit) continue;
-      const int np = tile_patches_1d(tx, g.ph, g.sh) * tile_patches_1d(ty, g.pw, g.sw);
-      const int cover = ((g.ph + g.sh - 1) / g.sh) * ((g.pw + g.sw - 1) / g.sw);
-      const double tiles = double((g.W + tx - 1) / tx) * ((g.H + ty - 1) / ty);
-      const double cta = 1200.0 * ((np + 31) / 32) * ((g.n + 159) / 160) +
-                         30.0 * cover * ((tx * ty + kCol2imThreads - 1) / kCol2imThreads) + 1500.0;
-      const double c = std::ceil(tiles / 296.0) * cta;  // two CTAs on each of 148 SMs
-      if (best.x == 0 || c < least) {
+      const double us = tile_us(g, L, num_sms, t);
+      if (us < least) {
         best = t;
-        least = c;
+        least = us;
       }
     }
   return best;
 }
 
-constexpr int kDirectThreads = 256;
-
-int col2im_num_tiles(const PatchGeom& g) {
-  const Tile t = pick_tile(g);
+int col2im_num_tiles(const PatchGeom& g, int L, int num_sms) {
+  const Tile t = pick_tile(g, L, num_sms);
   if (t.x == 0) return int((int64_t(g.W) * g.H + kDirectThreads - 1) / kDirectThreads);
-  return ((g.W + t.x - 1) / t.x) * ((g.H + t.y - 1) / t.y);
+  return ceil_div(g.W, t.x) * ceil_div(g.H, t.y);
 }
 
 // ix range covering x: ix*sh <= x < ix*sh + ph, 0 <= ix < nx
@@ -84,10 +102,10 @@ __device__ __forceinline__ int cover_lo(int x, int ext, int stride) {
 }
 __device__ __forceinline__ int cover_hi(int x, int stride, int npos) { return min(npos - 1, x / stride); }
 
-__global__ void __launch_bounds__(kCol2imThreads) col2im_kernel(const float* __restrict__ noisy, PatchGeom g, int TX, int TY,
-                                                     const float* __restrict__ D, int K, int L,
-                                                     const int32_t* __restrict__ idx, const float* __restrict__ coef,
-                                                     float* __restrict__ acc_out, double* __restrict__ partials) {
+__global__ void __launch_bounds__(kCol2imThreads)
+    col2im_kernel(const float* __restrict__ noisy, PatchGeom g, int TX, int TY, const float* __restrict__ D, int K,
+                  int L, const int32_t* __restrict__ idx, const float* __restrict__ coef,
+                  float* __restrict__ acc_out, double* __restrict__ partials) {
   extern __shared__ float xs[];
   __shared__ double red[32];
   const int tx0 = blockIdx.x * TX, ty0 = blockIdx.y * TY;
@@ -173,7 +191,7 @@ __global__ void __launch_bounds__(kCol2imThreads) col2im_kernel(const float* __r
 }
 
 // The same sums without shared memory, for patches too large for a tile's
-// covering patches to fit it: one thread per pixel forms the element of each
+// covering patches to fit it and for pixels that few patches cover: one thread per pixel forms the element of each
 // covering patch it needs (x_hat_p[r] = sum_s x_s d_s[r], the same FMA order
 // as col2im_kernel) and adds them in the same patch order, so the result is
 // identical; each block reduces its share of the lambda sum.
@@ -242,8 +260,8 @@ __global__ void blend_kernel(const float* __restrict__ noisy, PatchGeom g, const
 
 cudaError_t launch_col2im(const float* noisy, const PatchGeom& g, const float* dict, int K, int L,
                           const int32_t* idx, const float* coef, float* acc, double* partials, int* num_partials,
-                          cudaStream_t s) {
-  const Tile t = pick_tile(g);
+                          int num_sms, cudaStream_t s) {
+  const Tile t = pick_tile(g, L, num_sms);
   if (t.x == 0) {
     const int64_t blocks = (int64_t(g.W) * g.H + kDirectThreads - 1) / kDirectThreads;
     col2im_direct_kernel<<<unsigned(blocks), kDirectThreads, 0, s>>>(noisy, g, dict, K, L, idx, coef, acc, partials);
@@ -255,7 +273,7 @@ cudaError_t launch_col2im(const float* noisy, const PatchGeom& g, const float* d
     cudaError_t e = cudaFuncSetAttribute(col2im_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     if (e != cudaSuccess) return e;
   }
-  dim3 grid((g.W + t.x - 1) / t.x, (g.H + t.y - 1) / t.y);
+  dim3 grid(ceil_div(g.W, t.x), ceil_div(g.H, t.y));
   col2im_kernel<<<grid, kCol2imThreads, smem, s>>>(noisy, g, t.x, t.y, dict, K, L, idx, coef, acc, partials);
   *num_partials = int(grid.x * grid.y);
   return cudaGetLastError();

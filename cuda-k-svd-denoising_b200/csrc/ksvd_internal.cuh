@@ -243,8 +243,8 @@ cudaError_t launch_scatter_codes(const int32_t* sidx, const float* scoef, int L,
 // Image rebuild.
 cudaError_t launch_col2im(const float* noisy, const PatchGeom& g, const float* dict, int K, int L,
                           const int32_t* idx, const float* coef, float* acc, double* partials,
-                          int* num_partials, cudaStream_t s);
-int col2im_num_tiles(const PatchGeom& g);
+                          int* num_partials, int num_sms, cudaStream_t s);
+int col2im_num_tiles(const PatchGeom& g, int L, int num_sms);
 cudaError_t launch_blend(const float* noisy, const PatchGeom& g, const float* acc, const double* partials,
                          int num_partials, double sigma2, int speckle, float* out, double* lambda_dev,
                          cudaStream_t s);
