@@ -666,8 +666,8 @@ def main():
             "iteration_vs_bound": iter_bound,
             "phase_ms_one_step": {
                 name: phases[i] for i, name in (
-                    (7, "upd_setup"), (0, "upd_wait_prev_atom"), (1, "upd_load"), (2, "upd_pass"),
-                    (3, "upd_wait_partials"), (4, "upd_allreduce"), (5, "upd_coef_store"), (8, "omp_corr"),
+                    (7, "upd_setup"), (0, "upd_wait_prev_atom"), (1, "upd_issue_loads"), (2, "upd_columns_and_pass"),
+                    (3, "upd_sum_partials"), (4, "upd_normalise"), (5, "upd_coef_store"), (8, "omp_corr"),
                     (9, "omp_residual"), (10, "omp_io"), (11, "omp_rescore"), (12, "omp_cholesky"))},
             "counters_per_step": {k: (v if k.startswith("omp_") else v / max(args.steps, 1))
                                   for k, v in counters.items()},

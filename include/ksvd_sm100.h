@@ -71,12 +71,15 @@ typedef enum ksvd_status {
  * selected atom is the exact argmax either way; FP16 (11-bit significand,
  * exact power-of-two scaling per patch) gives an 8x narrower bound than BF16
  * and therefore far fewer re-scores.
- * The tensor-core forms apply for atoms <= 256 when the tile of 128 patches
- * and the 16-bit dictionary fit in shared memory; beyond that the FP32
- * kernels run (dictionary resident in shared memory when it fits, streamed
- * through it otherwise: atoms <= 1024). */
+ * The FP32 form takes the argmax of FP32 sums; on many patches an FP16
+ * correlation first narrows the atoms down to those that could hold it, with
+ * the same codes.
+ * The tensor cores serve up to 512 atoms (beyond 256 or so the 16-bit
+ * dictionary is streamed through shared memory), 16 atoms per patch and 512
+ * patch values; beyond that the FP32 kernels run (dictionary resident in
+ * shared memory when it fits, streamed through it otherwise: atoms <= 1024). */
 typedef enum ksvd_precision {
-  KSVD_PREC_FP32 = 0,         /* plain FP32 FMA                              */
+  KSVD_PREC_FP32 = 0,         /* plain FP32 sums                             */
   KSVD_PREC_BF16_RESCORE = 1, /* BF16 tensor cores + exact re-score         */
   KSVD_PREC_FP16_RESCORE = 2, /* FP16 tensor cores + exact re-score         */
   KSVD_PREC_BF16_LEARNED = 3  /* learned top-16 proposal (BF16 MLP on the
@@ -221,8 +224,8 @@ ksvd_status ksvd_profile_reset(ksvd_ctx* ctx);
 int64_t ksvd_launch_count(const ksvd_ctx* ctx);
 /* Wall time (ms) the first CTA of the persistent kernels spent per phase
  * while profiling at level 2 (since the last reset): update [7] slice set-up,
- * [0] wait for the previous atom, [1] column load, [2] local power pass (and
- * the arrival of the columns), [3] sum of the partials (waiting for the other
+ * [0] wait for the previous atom, [1] issue of the column loads, [2] local power
+ * pass (and the arrival of the columns), [3] sum of the partials (waiting for the other
  * CTAs'), [4] normalisation, [5] coefficients and residual store; OMP [8] correlation +
  * argmax, [9] residual update (least squares included for the FP32 kernels),
  * [10] tile load/store, [11] exact re-scores, [12] Cholesky append and solve
