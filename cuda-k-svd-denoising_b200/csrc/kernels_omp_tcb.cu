@@ -1,6 +1,6 @@
 // Batched OMP with the 16-bit tensor-core correlation for dictionaries too
 // large for the resident-dictionary kernel (kernels_omp_tc.cu): up to 512
-// atoms and patches of up to 256 values (CuBlasMatrixOmp::work,
+// atoms and patches of up to 512 values (CuBlasMatrixOmp::work,
 // cublas_matrix_omp.cu:107-402, with the correlation of :193-206 on the
 // tensor cores).
 //

@@ -104,7 +104,7 @@ cudaError_t launch_omp_tc(const float* patches, int64_t N, int n, const float* d
                           int64_t* fix_list = nullptr, unsigned long long* fix_count = nullptr);
 
 // OMP with the 16-bit tensor-core correlation for dictionaries beyond the
-// resident kernel (atoms <= 512, n <= 256): the 16-bit dictionary streams
+// resident kernel (atoms <= 512, n <= 512): the 16-bit dictionary streams
 // from `scratch` (omp_tcb_scratch_bytes, written by the launch).
 bool omp_tcb_supported(int n, int K, int L);
 size_t omp_tcb_scratch_bytes(int n, int K, TcForm form, int num_sms);
