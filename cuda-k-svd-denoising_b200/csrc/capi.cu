@@ -288,6 +288,27 @@ ksvd_status ksvd_init_dictionary(ksvd_ctx* c, const float* d_patches, int64_t N,
 namespace ksvd {
 namespace api {
 
+// The FP32 form on few patches: waves of the SIMT kernels' tiles (32 patches, one
+// an SM) up to which these are the faster ones.  A wave of the tensor-core kernels
+// takes four times the patches in one to two times the time.  Where the line lies
+// depends on whether the SIMT kernel keeps the dictionary in shared memory, and on
+// whether the tensor-core kernels can read rows in 16-byte pieces.  Measured (n = 25
+// to 484, 64 to 512 atoms, L = 2 to 16), SIMT time over tensor-core time:
+//   resident dictionary: 0.46 to 0.84 with one wave (64 values, 512 atoms, L = 5: 117 us
+//     against 172); with two, 0.84 to 1.3 where the tensor-core kernel is resident too
+//     (144, 256, 5: 206 / 212), else 0.73 to 1.09 within the limits on L below (49, 512,
+//     6: 188 / 219) and up to 1.6 beyond them (64, 300, 8: 302 / 232); 1.04 to 1.9 with three;
+//   streamed: with one wave 0.41 to 1.01 for up to 256 atoms (256, 256, 5: 250 / 316), 0.6 to
+//     0.93 where rows are not of 16-byte pieces (225, 512, 5: 399 / 477), 0.82 to 1.03 for
+//     100 values, 0.88 to 1.21 from 144 on (256, 512, 8: 621 / 565); with two 0.79 to 2.3.
+static int simt_max_waves(int n, int K, int L) {
+  const bool odd = (n & 3) != 0;
+  if (ksvd::omp_fp32_supported(n, K, L))
+    return (K <= 256 && ksvd::omp_tc_supported(n, K, L)) || L <= (odd ? 8 : n < 64 ? 6 : 3) ? 2 : 1;
+  if (!ksvd::omp_stream_supported(n, K, L)) return 0;
+  return K <= 256 || odd || n < 128 ? 1 : 0;
+}
+
 ksvd_status omp_form(ksvd_ctx* c, const float* d_patches, int64_t N, const float* d_dict, int32_t* d_idx,
                      float* d_coef, int precision, bool for_update) {
   const int n = c->p.patch_width_dim * c->p.patch_height_dim, K = c->p.atoms, L = c->p.omp_iter;
@@ -331,15 +352,8 @@ ksvd_status omp_form(ksvd_ctx* c, const float* d_patches, int64_t N, const float
   const ksvd::TcForm form = precision == KSVD_PREC_FP32           ? ksvd::TcForm::kFp32
                             : precision == KSVD_PREC_FP16_RESCORE ? ksvd::TcForm::kFp16
                                                                   : ksvd::TcForm::kBf16;
-  // The FP32 kernel of small dictionaries works on tiles of 32 patches, the
-  // tensor-core ones on tiles of 128: where one or two waves of the former cover
-  // the patches it is the faster one (8 x 8 patches, 256 atoms: 54 us a wave
-  // against 107; 16 x 16: 209 against 272 with the dictionary streamed; with 512
-  // atoms a wave takes 549 against 494, so the tensor cores always win).
   const int64_t simt_waves = (N + int64_t(32) * c->num_sms - 1) / (int64_t(32) * c->num_sms);
-  const bool simt = form == ksvd::TcForm::kFp32 && K <= 256 &&
-                    simt_waves <= (ksvd::omp_tc_supported(n, K, L) ? 2 : 1) &&
-                    (ksvd::omp_fp32_supported(n, K, L) || ksvd::omp_stream_supported(n, K, L));
+  const bool simt = form == ksvd::TcForm::kFp32 && simt_waves <= simt_max_waves(n, K, L);
   if (!simt && ksvd::omp_tc_supported(n, K, L)) {
     if (for_update) KSVD_TRY(fused_buffers());
     KSVD_CU(c,
