@@ -248,18 +248,20 @@ __global__ void __launch_bounds__(kSThreads, 1)
         if (sqrtf(nrm) < 1e-3f) done[tid] = 1;
       }
       // ---- argmax per patch --------------------------------------------------
-      // (N > 0; with a -1 in sight the compiler takes |x| > -1 to hold for a NaN
-      // too, and an atom's NaN would beat every number)
-      const float none = N > 0 ? -1.0f : 0.0f;
+      // (the first atom is tested against itself: with its start value -1 in sight
+      // the compiler takes |x| > -1 to hold for a NaN too, and that would beat
+      // every number)
       float bv[4];
       int bi[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        bv[j] = none;
-        bi[j] = 0x7fffffff;
+        const float v = fabsf(acc[0][j]);
+        const bool in = ag * APT < K && v == v;
+        bv[j] = in ? v : -1.0f;
+        bi[j] = in ? ag * APT : 0x7fffffff;
       }
 #pragma unroll
-      for (int i = 0; i < APT; ++i) {
+      for (int i = 1; i < APT; ++i) {
         const int a = ag * APT + i;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
