@@ -154,8 +154,8 @@ __host__ __device__ inline TcLayout tc_layout(int n, int K, int L) {
 
 // v, as a value of its own: what a part of a step derives from it is formed there.
 // From the plain thread index the compiler forms the addresses of every part ahead
-// of the loops and spills them (176 bytes of stack, 72 of spill loads a step; 48 so;
-// 100,000 patches of 12 x 12, 256 atoms: 769 -> 736 us in FP16, 954 -> 896 in FP32).
+// of the loops and spills them (68 bytes of spilled registers; 48 so; 100,000
+// patches of 12 x 12, 256 atoms: 769 -> 736 us in FP16, 954 -> 896 in FP32).
 KSVD_DEV int tc_own(int v) {
   asm volatile("" : "+r"(v));
   return v;
@@ -237,21 +237,12 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     asum[a] = sa;
     if constexpr (F32) atomicMax(&s_dmax, __float_as_uint(sq) & 0x7fffffffu);
   }
-  // F32 takes dictionaries of any scale: the 16-bit one is D / dscale (a power
-  // of two, atoms of norm below 1); out of the range where that is exact
-  // enough, dmax is infinite and every atom is scored
   float dmax = 1.0f, dscale = 1.0f;
   if constexpr (F32) {
     __syncthreads();
-    dmax = sqrtf(__uint_as_float(s_dmax));
-    if (dmax > 1e-15f && dmax < 1e15f) {
-      int e;
-      frexpf(dmax, &e);
-      dscale = ldexpf(1.0f, e);
-      dmax *= 1.0001f;
-    } else {
-      dmax = __int_as_float(0x7f800000);
-    }
+    const F32Scale t = f32_scale(s_dmax);
+    dmax = t.dmax;
+    dscale = t.scale;
     convert(1.0f / dscale);
   }
   fence_proxy_async_smem();

@@ -143,28 +143,6 @@ __host__ __device__ inline TbLayout tb_layout(int n, int K, int L) {
   return o;
 }
 
-// F32 takes dictionaries of any scale: the 16-bit one is D / scale (a power of
-// two, atoms of norm below 1); outside the range where that is exact enough,
-// `dmax` is infinite and every atom is scored.
-struct TbScale {
-  float dmax, scale;
-};
-
-__device__ __forceinline__ TbScale tb_scale(unsigned sq_bits) {
-  TbScale t;
-  t.dmax = sqrtf(__uint_as_float(sq_bits));
-  t.scale = 1.0f;
-  if (t.dmax > 1e-15f && t.dmax < 1e15f) {
-    int e;
-    frexpf(t.dmax, &e);
-    t.scale = ldexpf(1.0f, e);
-    t.dmax *= 1.0001f;
-  } else {
-    t.dmax = __int_as_float(0x7f800000);
-  }
-  return t;
-}
-
 // Bits of the largest |d_a|^2 (a NaN's are larger than any number's); a warp per atom.
 __global__ void tb_norm_kernel(const float* __restrict__ D, int K, int n, unsigned* __restrict__ sq_max) {
   const int a = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
@@ -184,7 +162,7 @@ template <bool F16>
 __global__ void tb_prep_kernel(const float* __restrict__ D, int K, int n, int Kp, int np16,
                                unsigned char* __restrict__ Bg, float* __restrict__ asum,
                                const unsigned* __restrict__ sq_max) {
-  const float dinv = sq_max ? 1.0f / tb_scale(*sq_max).scale : 1.0f;
+  const float dinv = sq_max ? 1.0f / f32_scale(*sq_max).scale : 1.0f;
   const int nkc = np16 / 8;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < Kp * nkc; t += gridDim.x * blockDim.x) {
     const int a = t / nkc, kc = t - a * nkc;
@@ -275,7 +253,7 @@ __global__ void __launch_bounds__(kTbThreads, 1)
   int nscored = 0;
   float dmax = 1.0f, dscale = 1.0f;
   if constexpr (F32) {
-    const TbScale t = tb_scale(*sq_max);
+    const F32Scale t = f32_scale(*sq_max);
     dmax = t.dmax;
     dscale = t.scale;
   }
