@@ -26,7 +26,7 @@
 // FP32 value within both rounding errors are scored with that very sum, so the
 // codes are the ones of kernels_omp.cu.  The tile keeps the FP32 residual in
 // shared memory in the place of the patches, which are read again from L2.
-// (2048 x 2048 image, 12 x 12 patches, 256 atoms, L = 5: 4.3 ms, 7.7 with the
+// (2048 x 2048 image, 12 x 12 patches, 256 atoms, L = 5: 3.66 ms, 7.7 with the
 // SIMT correlation, which is bound by the FP32 pipe; 1.4 atoms scored per patch
 // and step.  Bound now by the latency of the epilogue, like the 16-bit forms.)
 #include <cuda_bf16.h>

@@ -54,13 +54,17 @@ struct LanePlan {
   double total_ms = 0.0;
 };
 
-// Sweep time of one image on w CTAs (ms), a model measured on B200 with the
-// update kernel (one image at a time on every SM, 64 images of 8 x 8 to
-// 22 x 22 patches): per atom a latency floor of 11 + 0.025 n us (the
-// all-reduces and the hand-over between atoms), plus the local passes over
-// the atom's columns, 8.6e-4 us per column and feature spread over the w
-// CTAs, five times dearer for columns beyond a CTA's shared-memory capacity
-// (streamed from memory on every power step).
+// Cost of one image's sweep on w CTAs (ms), what plans are compared by: per atom
+// a latency floor of 11 + 0.025 n us (the all-reduces and the hand-over between
+// atoms), plus the local passes over the atom's columns, 8.6e-4 us per column
+// and feature spread over the w CTAs, five times dearer for columns beyond a
+// CTA's shared-memory capacity (streamed from memory on every power step).
+// The constants were fitted to an earlier form of the update kernel, which took
+// a third longer an atom, and are no longer its times (64 uneven images: 159 ms
+// modelled, 133 measured; 24 images: 40 and 52).  Fitted to the present kernel,
+// one image at a time on 18 to 148 CTAs (9.9 + 0.0137 n us, 7.4e-4 us, streamed
+// columns no dearer), they chose more and narrower lanes, whose streamed columns
+// side by side take longer than one image alone shows: 169 ms and 78 ms.
 double sweep_model_ms(const LaneShape& s, int w) {
   const double E = s.N * s.L / double(s.K);  // entries per atom
   const double floor_us = 11.0 + 0.025 * s.n;
